@@ -533,9 +533,11 @@ struct mxg_engine {
     unsigned *d_status = nullptr;
     unsigned long long *d_step = nullptr;
     double *d_partials = nullptr, *d_energy = nullptr;
-    int energy_blocks = 64;
+    int energy_blocks = 148;
+    unsigned *d_red_done = nullptr;     // finished blocks of the energy reduction and of the kinetic energy pass
     bool has_dpd = false;
     bool has_sb = false;                // a type has a Berendsen, random or friction force
+    bool has_berendsen = false, has_persist = false;  // a type has a Berendsen; a random or friction force
     bool has_walls = false;             // a type has a wall potential
     int nlarge = 0;                     // large particles (radius > cutoff)
     float4 *d_large_x = nullptr, *d_large_v = nullptr;
@@ -545,7 +547,7 @@ struct mxg_engine {
     bool has_cuboid_forces = false;     // a cuboid exists and a type has a cuboid potential
     DevCuboid *d_cuboids = nullptr;
     bool has_body() const { return has_walls || nlarge > 0 || has_cuboid_forces; }
-    double *d_type_ke = nullptr;
+    double *d_type_ke = nullptr, *d_ke_partials = nullptr;
     float4 *d_persist = nullptr;
     int integrator = 0;                 // 0 forward Euler, 1 Runge-Kutta 4 (engine.h EngineIntegrator)
     int force_layout = 0;               // the buffer whose slot order the force array follows
@@ -792,12 +794,19 @@ struct mxg_engine {
         return bv;
     }
 
+    /* What the single-body forces read; redraw: the step's first force pass. */
+    void enqueue_singlebody_prep(const EngineView &v, bool redraw) {
+        if (!has_sb) return;
+        launch_singlebody_prep(v, has_berendsen ? d_type_ke : nullptr, d_ke_partials, d_red_done + 1,
+                               redraw && has_persist ? d_persist : nullptr, stream);
+    }
+
     /* The force pass alone (engine_force): the bonded kernel, or the combine
      * kernel when there are no bonded interactions, adds the received planes. */
     void enqueue_force(int b) {
         force_layout = b;
         const EngineView v = view(b);
-        if (has_sb) launch_singlebody_prep(v, ntypes, d_type_ke, d_persist, false, stream);
+        enqueue_singlebody_prep(v, false);
         if (has_body()) launch_body(v, d_body_f, stream);
         launch_force(v, has_dpd, force_grid, !has_bonded(), stream);
         if (has_bonded()) launch_bonded(v, bonded_view(), stream);
@@ -841,7 +850,7 @@ struct mxg_engine {
         }
         const EngineView v = view(b);
         mark(0);
-        if (has_sb) launch_singlebody_prep(v, ntypes, d_type_ke, d_persist, true, stream);
+        enqueue_singlebody_prep(v, true);
         if (has_body()) launch_body(v, d_body_f, stream);
         mark(1);
         launch_force(v, has_dpd, force_grid, false, stream);
@@ -873,7 +882,7 @@ struct mxg_engine {
         const EngineView v = view(b);
         for (int stage = 0; stage < 4; ++stage) {
             // persistent random forces are redrawn in the first stage only (INTEGRATOR_UPDATE_PERSISTENTFORCE)
-            if (has_sb) launch_singlebody_prep(v, ntypes, d_type_ke, d_persist, stage == 0, stream);
+            enqueue_singlebody_prep(v, stage == 0);
             if (has_body()) launch_body(v, d_body_f, stream);
             launch_force(v, has_dpd, force_grid, false, stream);
             if (has_bonded()) launch_bonded(v, bonded_view(), stream);
@@ -1198,7 +1207,7 @@ int mxg_engine::start(cudaStream_t st) {
         if (k >= 0) dpd_pure = false;
     h_pot_idx = hpidx;
     const std::vector<float4> hdpd = dpd_records(hp);
-    has_sb = false;
+    has_sb = has_berendsen = has_persist = false;
     has_walls = false;
     has_cuboid_forces = false;
     std::vector<DevType> ht(ntypes);
@@ -1228,6 +1237,8 @@ int mxg_engine::start(cudaStream_t st) {
             d.sb_steps = std::max(1, (int)std::ceil(dur / dt));  // durration_steps (MxForce.cpp:403,417)
         }
         if (ti.sb_kind) has_sb = true;
+        if (ti.sb_kind == 2) has_berendsen = true;
+        if (ti.sb_kind == 3 || ti.sb_kind == 4) has_persist = true;
         if (is_large[a]) {
             d.large = 1;
             d.flags |= (1u << 2) | (1u << 3) | (1u << 4);  // never integrated (not in any cell of the reference)
@@ -1407,6 +1418,8 @@ int mxg_engine::start(cudaStream_t st) {
     rc |= alloc(&d_cuboids, hcub.size());
     rc |= alloc(&d_types, ht.size());
     rc |= alloc(&d_type_ke, ht.size());
+    rc |= alloc(&d_ke_partials, has_berendsen ? ht.size() * type_ke_blocks(nparts) : 0);
+    rc |= alloc(&d_red_done, 2);
     rc |= alloc(&d_persist, (size_t)nparts);
     rc |= alloc(&d_spaces, hs.size());
     rc |= alloc(&d_axes, 1);
@@ -1463,6 +1476,7 @@ int mxg_engine::start(cudaStream_t st) {
     if (smax > 0) CUDA_TRY(cudaMemsetAsync(d_rate, 0, sizeof(float) * (size_t)nparts * smax, stream));
     CUDA_TRY(cudaMemsetAsync(d_force, 0, sizeof(float4) * std::max(1, nparts), stream));
     CUDA_TRY(cudaMemsetAsync(d_persist, 0, sizeof(float4) * std::max(1, nparts), stream));
+    CUDA_TRY(cudaMemsetAsync(d_red_done, 0, 2 * sizeof(unsigned), stream));
     CUDA_TRY(cudaMemsetAsync(d_type_ke, 0, sizeof(double) * ht.size(), stream));
     if ((rc = upload(d_pos[0], hpos, stream)) || (rc = upload(d_vel[0], hvel, stream)) ||
         (rc = upload(d_cell_of[0], hcell_of, stream)) || (rc = upload(d_cell_start[0], hstart, stream)) ||
@@ -2336,7 +2350,7 @@ int mxg_engine_energy(mxg_engine *e, double *epot, double *ekin, double *virial9
     if (!e) return MXG_ERR_NULL;
     if (!e->started) return MXG_ERR_STATE;
     launch_energy(e->nitems, e->d_epot_cell, e->nparts, e->has_bonded() ? e->d_ebond_slot : nullptr,
-                  e->has_body() ? e->d_body_e : nullptr, e->d_vel[e->cur], e->d_pos[e->cur], e->d_types, e->d_partials, e->energy_blocks, e->d_energy,
+                  e->has_body() ? e->d_body_e : nullptr, e->d_vel[e->cur], e->d_pos[e->cur], e->d_types, e->d_partials, e->energy_blocks, e->d_red_done, e->d_energy,
                   e->stream);
     double out[2];
     CUDA_TRY(cudaMemcpyAsync(out, e->d_energy, sizeof(out), cudaMemcpyDeviceToHost, e->stream));
@@ -2464,7 +2478,7 @@ int mxg_engine_energy_async(mxg_engine *e, double *host_out2) {
     if (!e || !host_out2) return MXG_ERR_NULL;
     if (!e->started) return MXG_ERR_STATE;
     launch_energy(e->nitems, e->d_epot_cell, e->nparts, e->has_bonded() ? e->d_ebond_slot : nullptr,
-                  e->has_body() ? e->d_body_e : nullptr, e->d_vel[e->cur], e->d_pos[e->cur], e->d_types, e->d_partials, e->energy_blocks, e->d_energy,
+                  e->has_body() ? e->d_body_e : nullptr, e->d_vel[e->cur], e->d_pos[e->cur], e->d_types, e->d_partials, e->energy_blocks, e->d_red_done, e->d_energy,
                   e->stream);
     CUDA_TRY(cudaMemcpyAsync(host_out2, e->d_energy, 2 * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
     return MXG_OK;

@@ -13,10 +13,12 @@ int force_variants();
 void launch_group_metrics(const EngineView &v, const int *ids, int n, const int *slot_of_id, double *out,
                           cudaStream_t st);
 void launch_sort_bounds(const EngineView &v, cudaStream_t st);
-/* Before a force pass: the per-type kinetic energy (Berendsen) and, when redraw is set (the
- * step's first force pass), the persistent random forces due at this step. */
-void launch_singlebody_prep(const EngineView &v, int ntypes, double *type_ke, float4 *persist, bool redraw,
-                            cudaStream_t st);
+/* Before a force pass: the kinetic energy of the types with a Berendsen force (type_ke null: none;
+ * ke_partials: type_ke_blocks() doubles per type, ke_done: a zeroed counter) and, when persist is
+ * not null (the step's first force pass), the persistent random forces due at this step. */
+int type_ke_blocks(int nparts);
+void launch_singlebody_prep(const EngineView &v, double *type_ke, double *ke_partials, unsigned *ke_done,
+                            float4 *persist, cudaStream_t st);
 void launch_virial_reduce(const double *partials, int nwarps, double *out9, cudaStream_t st);
 /* out9 += the virial of the bonded terms (nb bonds, nx exclusions, na angles, nd dihedrals) of the
  * current positions; partials: nblocks * 9 doubles of scratch */
@@ -68,10 +70,11 @@ void launch_load_order(const EngineView &v, const LoadView &ld, const int *count
  * order the forces were computed in */
 void launch_unload(const EngineView &v, const float4 *force_ids, double *x, float *vel, float *f, int *cell,
                    float *xrel, cudaStream_t st);
-/* ebond_slot, body_e: per-slot bonded and wall energies of the last pass (null when absent) */
+/* ebond_slot, body_e: per-slot bonded and wall energies of the last pass (null when absent); partials:
+ * 2 * nblocks doubles, done: a zeroed counter */
 void launch_energy(int ncells, const double *epot_cell, int nparts, const double *ebond_slot, const double *body_e,
                    const float4 *vel, const float4 *pos, const DevType *types, double *partials, int nblocks,
-                   double *out, cudaStream_t st);
+                   unsigned *done, double *out, cudaStream_t st);
 
 /* The pairwise bond constructor's pair search (mxg_pairs.cu): pairs (a, b), b < a, of the list ids
  * with |x_a - x_b|^2 <= cutoff^2 in global FP32 coordinates (no periodic image) whose type pair has a
