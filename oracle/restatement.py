@@ -3,8 +3,8 @@
 TEST INFRASTRUCTURE ONLY. Computes the nonbonded forces and energy of a
 configuration in FP32 (reference operation order) or FP64 on the same FP32
 table coefficients. Tables come from the reference's own table builder
-(oracle/_ref/libmxref.so) when it is built, else from the committed golden
-tables.
+(oracle/_ref/libmxref.so) when it is built, else from this package's builder
+(bit-identical to the committed golden tables, tests/test_tables.py).
 """
 import ctypes
 import os
@@ -51,6 +51,8 @@ def lib():
 def reference_table(kind, params):
     """(info dict, coefficients) from the reference's table builder (in process)."""
     from . import refengine
+    if not refengine.available():
+        return _package_table(kind, params)
     L = ctypes.PyDLL(refengine.LIB)
     vp, cd = ctypes.c_void_p, ctypes.c_double
     if kind == "dpd":
@@ -79,6 +81,20 @@ def reference_table(kind, params):
         L.mxref_potential_coeffs(vp(p), coef.ctypes.data_as(ctypes.POINTER(ctypes.c_float)), coef.size)
     return dict(kind=k.value, flags=fl.value, n=n.value, alpha=np.array(a4[:3], dtype=np.float32), a=a.value,
                 b=b.value, r0p1=r0.value), coef
+
+
+def _package_table(kind, params):
+    """The same from this package's table builder, whose tables tests/test_tables.py holds bit for
+    bit to the committed golden ones (for where the reference's sources are not at hand)."""
+    from mechanica_b200 import EngineError, workloads
+    try:
+        p = workloads.make_potential(kind, [float(q) for q in params])
+    except EngineError:
+        return None, None
+    i = p._info()
+    coef = p.coefficients if i["kind"] == 0 else np.zeros(8, dtype=np.float32)
+    return dict(kind=i["kind"], flags=i["flags"], n=i["n"], alpha=i["alpha"][:3], a=i["a"], b=i["b"],
+                r0p1=i["r0_plusone"]), coef
 
 
 def cell_origins(dim, cdim, origin=(0.0, 0.0, 0.0)):
