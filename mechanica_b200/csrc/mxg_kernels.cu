@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, TS::kBlocks) force_kernel
  * threads read consecutive words), then a tree over the rows; the first kComp threads return
  * their component's sum. The order of the additions is fixed. One thread a component would
  * walk the rows as one chain of dependent loads and FP64 additions: 534 us for the pair
- * virial's 9,472 rows against 5 us. */
+ * virial's 9,472 rows against 14 us. */
 template <int kComp, int kRows>
 __device__ __forceinline__ double sum_rows(const double *__restrict__ rows, int n) {
     __shared__ double part[kComp * kRows];
@@ -1390,7 +1390,7 @@ __device__ __forceinline__ bool last_block(unsigned *done) {
  * partial per type; the block that finishes last adds the partials, so the order is fixed.
  * Bound: latency of one load and the last block's pass (the data are 32 B a particle). One
  * block a type over all particles took 42.7 us at 10,000 particles and 243 us at 61,000, this
- * 5.0 and 5.9 us. */
+ * 6.2 us at both. */
 constexpr int kKeThreads = 256, kKePer = 4;
 __global__ void __launch_bounds__(kKeThreads) type_ke_kernel(EngineView v, double *partials, unsigned *done, double *out) {
     int type[kKePer];
@@ -2388,9 +2388,10 @@ constexpr int kScanTile = 1024 * kScanPer;
 __device__ __forceinline__ int scan_slot(int i) { return i + i / kScanPer; }
 __global__ void __launch_bounds__(1024) load_scan_kernel(const int *__restrict__ count, int ncells, int *start,
                                                          int *count_out, const int *err) {
+    // count_out and err may be null
     __shared__ int tile[kScanTile + kScanTile / kScanPer];
     __shared__ int warp_sums[32];
-    if (*err) return;
+    if (err && *err) return;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     int carry = 0;
     for (int t0 = 0; t0 < ncells; t0 += kScanTile) {
@@ -2400,7 +2401,7 @@ __global__ void __launch_bounds__(1024) load_scan_kernel(const int *__restrict__
             const int i = k * 1024 + tid;
             const int ci = i < m ? count[t0 + i] : 0;
             tile[scan_slot(i)] = ci;
-            if (i < m) count_out[t0 + i] = ci;
+            if (count_out && i < m) count_out[t0 + i] = ci;
         }
         __syncthreads();
         int c[kScanPer], run = 0;
@@ -2798,6 +2799,10 @@ void launch_load_order(const EngineView &v, const LoadView &ld, const int *count
         if (vel_ready) cudaStreamWaitEvent(st, vel_ready, 0);
         load_vel_kernel<<<(ld.n + 255) / 256, 256, 0, st>>>(ld, slot_of_id, vel_out);
     }
+}
+
+void launch_scan(const int *count, int n, int *start, cudaStream_t st) {
+    load_scan_kernel<<<1, 1024, 0, st>>>(count, n, start, nullptr, nullptr);
 }
 
 void launch_unload(const EngineView &v, const float4 *force_ids, double *x, float *vel, float *f, int *cell,

@@ -66,6 +66,8 @@ void launch_load_place(const EngineView &v, const LoadView &ld, int *count, cuda
 void launch_load_order(const EngineView &v, const LoadView &ld, const int *count, int *start, int *count_out,
                        float4 *pos_out, float4 *vel_out, int *cell_out, int *slot_of_id, cudaEvent_t vel_ready,
                        cudaStream_t st);
+/* Exclusive scan of count[n] into start[n + 1] (start[n]: the total) */
+void launch_scan(const int *count, int n, int *start, cudaStream_t st);
 /* engine_unload's arrays by id on the device (any output may be null); force_ids: the velocities of the slot
  * order the forces were computed in */
 void launch_unload(const EngineView &v, const float4 *force_ids, double *x, float *vel, float *f, int *cell,
