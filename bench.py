@@ -55,7 +55,7 @@ F_INT_TABLE = 44
 
 # the sources that decide what a force launch does: its kernels and device structures, the host
 # engine that builds its work items, tables and launch configuration, and the build flags
-FORCE_SOURCES = ("mechanica_b200/csrc/mxg_kernels.cu", "mechanica_b200/csrc/mxg_kernels.h",
+FORCE_SOURCES = ("mechanica_b200/csrc/mxg_kernels.cu", "mechanica_b200/csrc/mxg_force.cu", "mechanica_b200/csrc/mxg_kernels.h",
                  "mechanica_b200/csrc/mxg_device.cuh", "mechanica_b200/csrc/mxg_engine.cpp",
                  "mechanica_b200/csrc/potential_table.cpp", "mechanica_b200/csrc/potential_table.h",
                  "mechanica_b200/build.py")

@@ -76,7 +76,7 @@ struct DevPot {          // one per potential, 64 B
     float a, b, r0_plusone;
     float dpd_alpha, dpd_gamma, dpd_sigma, dpd_delta;  // delta = 1/sqrt(dt) as the reference keeps it
     float a2;            // a*a (float)
-    float pad;
+    float inv_b;         // 1 / b
 };
 
 struct DevType {
@@ -135,6 +135,16 @@ struct DevSpace {        // one per replica
     float sort_dscale;   // SHRT_MAX / (2 |h|)
     int dmaxdist;        // 2 + dscale * cutoff
     int pad2;
+    // cell-pair shifts per axis, as the task list has them: between neighbours, and between the first
+    // and the last cell across the periodic face; axes periodic (bits)
+    float sh[3], shw[3];
+    int periodic;
+    // the column force kernel's position unit (a power of two, 2^-27 to 2^-26 of a cell edge) and its
+    // inverse; whether particles may lie outside their cells (Runge-Kutta stages)
+    float col_unit, col_scale;
+    float near_cut;          // relative width in r^2 within which its decisions at a cutoff are left to the
+                             // reference's arithmetic
+    int off_cell;
     double dt_d;         // the engine's dt in double (species integration)
     double cutoff_d;     // the space's cutoff in double (flux weight)
 };
@@ -229,7 +239,8 @@ struct EngineView {      // everything a kernel needs, passed by value
     const unsigned long long *step;  // device step counter
     const SortAxes *axes;
     int2 *sort_bounds;               // per cell and sort axis: (min key, max key)
-    double *epot_cell;       // per force work item: nonbonded energy of the last force pass
+    int *cell_near;                  // per cell: a particle near a face, by the axes' keys (cell_sort_bounds)
+    double *epot_cell;       // per force work item, then kColumnParts per column item: energy of the last force pass
     unsigned *status;
     unsigned long long *pair_stats;  // non-null only for the statistics launch
     double *virial_partials;         // non-null only for the virial launch: [warp][6]
@@ -255,10 +266,18 @@ struct EngineView {      // everything a kernel needs, passed by value
     int nitems;
     const DevCuboid *cuboids;  // static cuboids (all replicas)
     int ncuboids;
+    // per replica and type pair, the column kernel's record of the pair's potential and, if any is summed, of
+    // its second one: (a^2, m, c, b), (alpha0, alpha1, alpha2, interval count << 20 | first coefficient / 8)
+    // of a table at s = m r + c; (a^2, cutoff, 1 / cutoff, radii sum if shifted), (alpha, gamma, sigma delta,
+    // -1) of a DPD potential; a last word of -2: none
+    const float4 *pair_rec, *pair_rec2;
     const float4 *dpd_pair;  // DPD-only kernel, per replica and type pair: (rc, alpha, gamma, sigma delta),
                              // (a^2, a, 1/rc, alpha + sigma delta); null otherwise
     int *ovf_list;           // movers beyond their destination's bucket this step: old slot (capacity nparts)
     int *ovf_count;          // entries of ovf_list (re-armed by the re-binning launch)
+    // the column force kernel (spaces it applies to; the others' cells are in items)
+    const int4 *col_items;   // (first cell of a column, first group of 32 particles, group step, cells along z)
+    int ncol_items;
     int *chunk_delta;        // per chunk of 1 << kChunkShift cells: movers in minus movers out this step
 };
 

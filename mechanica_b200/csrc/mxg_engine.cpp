@@ -367,6 +367,45 @@ struct Space {
         return MXG_OK;
     }
 
+    /* The shifts between neighbouring cells along axis k as getsid forms them: a within the box, b
+     * across the periodic face. False when they depend on the cell (their rounding). */
+    bool axis_shifts(int k, float &a, float &b) const {
+        int at[3] = {0, 0, 0}, next[3] = {0, 0, 0};
+        a = b = (float)h[k];
+        for (int l = 0; l < cdim[k]; ++l) {
+            at[k] = l;
+            next[k] = (l + 1) % cdim[k];
+            const bool wraps = l + 1 == cdim[k];
+            if (wraps && (cdim[k] < 3 || !((period >> k) & 1))) continue;
+            int ci = cellid(at[0], at[1], at[2]), cj = cellid(next[0], next[1], next[2]);
+            const int c0 = ci;
+            float shift[3];
+            getsid(ci, cj, shift);
+            const float x = ci == c0 ? shift[k] : -shift[k];
+            if (wraps)
+                b = x;
+            else if (l == 0)
+                a = x;
+            else if (x != a)
+                return false;
+        }
+        return true;
+    }
+
+    /* Whether the column force kernel covers this space: cubic cells no smaller than the cutoff, so that
+     * every pair of neighbouring cells is one task and the per-pair projection test, whichever the
+     * pruning mode, drops no pair inside the cutoff. */
+    bool columns_apply(double cutoff) const {
+        if (!(h[0] == h[1] && h[1] == h[2])) return false;
+        for (int k = 0; k < 3; ++k) {
+            float a, b;
+            if (std::ceil(cutoff * ih[k]) != 1.0) return false;
+            if (((period >> k) & 1) && cdim[k] < 3) return false;
+            if (!axis_shifts(k, a, b)) return false;
+        }
+        return true;
+    }
+
     /* space_addpart's placement plus the first shuffle: local cell index and
      * cell-relative float position. */
     int place(const double *x, int &cell, float *xr) const {
@@ -487,17 +526,24 @@ struct mxg_engine {
     bool dpd_pure = false;              // every pair potential DPD, no summed second term, no Philox
     int *d_cell_planes = nullptr;       // planes summed into each cell's forces
     int nitems = 0;
+    int4 *d_all_items = nullptr;        // the cell kernel's items with every cell (pair counts and virial)
+    int nall_items = 0;
+    int4 *d_col_items = nullptr;        // the column force kernel's items
+    int ncol_items = 0;
+    int col_split = 1;                  // warps per group of the column force kernel
     DevPot *d_pots = nullptr;
     float *d_coef = nullptr;
     int *d_pot_idx = nullptr;
     int *d_pot_idx2 = nullptr;   // second summed potential per type pair, or -1
+    float4 *d_pair_rec = nullptr, *d_pair_rec2 = nullptr;  // column kernel: two records per replica and type pair
     float4 *d_dpd_pair = nullptr;  // DPD-only kernel: two records per replica and type pair
-    std::vector<int> h_pot_idx;    // the device's potential index per replica and type pair
+    std::vector<int> h_pot_idx, h_pot_idx2;  // the device's potential indices per replica and type pair
     bool has_second = false;
     DevType *d_types = nullptr;
     DevSpace *d_spaces = nullptr;
     SortAxes *d_axes = nullptr;
     int2 *d_sort_bounds = nullptr;
+    int *d_cell_near = nullptr;
     double *d_epot_cell = nullptr, *d_ebond_slot = nullptr;
     DevBond *d_bonds = nullptr;
     unsigned *d_bond_flags = nullptr;
@@ -546,6 +592,24 @@ struct mxg_engine {
     float4 *d_body_f = nullptr;         // per slot: wall and large-particle force of the pass
     bool has_cuboid_forces = false;     // a cuboid exists and a type has a cuboid potential
     DevCuboid *d_cuboids = nullptr;
+    /* warps per group of the column kernel: the default, or pinned by the variant */
+    int column_split() const {
+        return force_variant == 0 ? col_split : force_variant == 1 ? 1 : force_variant == 2 ? 4 : 8;
+    }
+    /* blocks the force kernels' work items can occupy */
+    int max_force_grid() const { return std::max((nitems + kWarpsPerBlock - 1) / kWarpsPerBlock, ncol_items); }
+    /* What the statistics and virial launches run on: the cell kernel over every cell (each pair once, in
+     * the reference's arithmetic). */
+    EngineView all_cells_view() const {
+        EngineView v = view(cur);
+        v.items = d_all_items;
+        v.nitems = nall_items;
+        v.ncol_items = 0;
+        v.item_order = nullptr;
+        return v;
+    }
+    /* the force kernels leave sums or forces that total_force still has to add */
+    bool needs_combine() const { return nitems > 0 || has_body() || has_sb; }
     bool has_body() const { return has_walls || nlarge > 0 || has_cuboid_forces; }
     double *d_type_ke = nullptr, *d_ke_partials = nullptr;
     float4 *d_persist = nullptr;
@@ -585,6 +649,46 @@ struct mxg_engine {
         return out;
     }
 
+    /* The column kernel's records of the type pairs' potentials pidx (see EngineView::pair_rec). */
+    std::vector<float4> pair_records(const std::vector<DevPot> &hp, const std::vector<int> &pidx) const {
+        std::vector<float4> out(std::max<size_t>(1, 2 * pidx.size()));
+        auto as_float = [](int x) {
+            float f;
+            memcpy(&f, &x, 4);
+            return f;
+        };
+        const int tt = ntypes * ntypes;
+        for (size_t k = 0; k < pidx.size(); ++k) {
+            out[2 * k] = make_float4(0.f, 0.f, 0.f, -1e30f);  // no distance is in range
+            out[2 * k + 1] = make_float4(0.f, 0.f, 0.f, as_float(-2));
+            if (pidx[k] < 0) continue;
+            const DevPot &d = hp[pidx[k]];
+            const int a = (int)(k % tt) / ntypes, b = (int)(k % tt) % ntypes;
+            const float rsum = (float)types[a].radius + (float)types[b].radius;
+            if (d.kind == kKindDPD) {
+                const bool shifted = d.flags & kFlagShifted;
+                const float cut = shifted ? d.b + rsum : d.b;
+                out[2 * k] = make_float4(d.a2, cut, 1.0f / cut, shifted ? rsum : 0.f);
+                out[2 * k + 1] = make_float4(d.dpd_alpha, d.dpd_gamma, d.dpd_sigma * d.dpd_delta, as_float(-1));
+            } else {
+                const bool scaled = d.flags & kFlagScaled, shifted = !scaled && (d.flags & kFlagShifted);
+                out[2 * k] = make_float4(d.a2, scaled ? 1.0f / rsum : 1.0f, shifted ? d.r0_plusone - rsum : 0.f, d.b);
+                out[2 * k + 1] = make_float4(d.alpha0, d.alpha1, d.alpha2, as_float((int)((unsigned)d.n << 20 | (unsigned)(d.coef_off / kChunk))));
+            }
+        }
+        return out;
+    }
+
+    /* Whether the records can hold every table (interval counts and places in the coefficient pool). */
+    bool records_hold() const {
+        size_t intervals = 0;
+        for (const auto &t : pots) {
+            if (t.n >= 1 << 11) return false;
+            intervals += t.c.size() / kChunk;
+        }
+        return intervals < (size_t)1 << 20;
+    }
+
     /* Device form of the potentials: one DevPot each and the pooled coefficients. */
     void pot_arrays(std::vector<DevPot> &hp, std::vector<float> &coef) {
         hp.clear();
@@ -604,6 +708,7 @@ struct mxg_engine {
             d.b = t.b;
             d.r0_plusone = t.r0_plusone;
             d.a2 = t.a * t.a;
+            d.inv_b = 1.0f / t.b;
             d.dpd_alpha = t.dpd_alpha;
             d.dpd_gamma = t.dpd_gamma;
             d.dpd_sigma = t.dpd_sigma;
@@ -664,6 +769,16 @@ struct mxg_engine {
         const bool cubic = sp.h[0] == sp.h[1] && sp.h[1] == sp.h[2];
         S.prune = pruning == 2 ? 0 : (2 | ((pruning == 1 || !cubic) ? 1 : 0));
         S.dmaxdist = sp.dmaxdist(cutoff);
+        for (int k = 0; k < 3; ++k) sp.axis_shifts(k, S.sh[k], S.shw[k]);
+        S.periodic = (int)sp.period;
+        int exponent = 0;
+        std::frexp((float)sp.h[2], &exponent);  // h in [2^(e-1), 2^e)
+        S.col_scale = std::ldexp(1.0f, 27 - exponent);
+        S.col_unit = std::ldexp(1.0f, exponent - 27);
+        // displacements round at two cell edges in the reference, here at 2^-24 of themselves: twice that,
+        // relative to the cutoff, for r^2, with a factor of two to spare
+        S.near_cut = (float)(4.0 * 2.4e-7 * 2.0 * std::max(cutoff, sp.h[2]) / cutoff);
+        S.off_cell = integrator == 1 ? 1 : 0;
         S.sort_bias = sp.sort_bias();
         S.sort_dscale = sp.sort_dscale();
         return S;
@@ -737,6 +852,7 @@ struct mxg_engine {
         v.step = d_step;
         v.axes = d_axes;
         v.sort_bounds = d_sort_bounds;
+        v.cell_near = d_cell_near;
         v.epot_cell = d_epot_cell;
         v.status = d_status;
         v.pair_stats = nullptr;
@@ -753,6 +869,8 @@ struct mxg_engine {
         v.dpd_pure = dpd_pure ? 1 : 0;
         v.force_variant = force_variant;
         v.nitems = nitems;
+        v.col_items = d_col_items;
+        v.ncol_items = ncol_items;
         v.planes = d_planes;
         v.body_e = has_body() ? d_body_e : nullptr;
         v.body_f = has_body() ? d_body_f : nullptr;
@@ -764,6 +882,8 @@ struct mxg_engine {
         v.cuboids = d_cuboids;
         v.ncuboids = has_cuboid_forces ? (int)cuboids.size() : 0;
         v.dpd_pair = dpd_pure ? d_dpd_pair : nullptr;
+        v.pair_rec = d_pair_rec;
+        v.pair_rec2 = d_pair_rec2;
         v.chunk_delta = d_chunk_delta[b];
         v.ovf_list = d_ovf_list;
         v.ovf_count = d_ovf_count;
@@ -808,7 +928,7 @@ struct mxg_engine {
         const EngineView v = view(b);
         enqueue_singlebody_prep(v, false);
         if (has_body()) launch_body(v, d_body_f, stream);
-        launch_force(v, has_dpd, force_grid, !has_bonded(), stream);
+        launch_force(v, has_dpd, force_grid, column_split(), !has_bonded(), stream);
         if (has_bonded()) launch_bonded(v, bonded_view(), stream);
         if (has_fluxes) launch_fluxes(v, species_view(), stream);
     }
@@ -853,13 +973,13 @@ struct mxg_engine {
         enqueue_singlebody_prep(v, true);
         if (has_body()) launch_body(v, d_body_f, stream);
         mark(1);
-        launch_force(v, has_dpd, force_grid, false, stream);
+        launch_force(v, has_dpd, force_grid, column_split(), false, stream);
         mark(2);
         if (has_bonded()) launch_bonded(v, bonded_view(), stream);
         if (has_fluxes) launch_fluxes(v, species_view(), stream);
         mark(3);
-        launch_integrate(v, d_pos[b], d_vel[b], d_new_cell, d_in_count[b], d_in_list, d_out_count[b], !has_bonded(),
-                         stream);
+        launch_integrate(v, d_pos[b], d_vel[b], d_new_cell, d_in_count[b], d_in_list, d_out_count[b],
+                         !has_bonded() && needs_combine(), stream);
         if (has_fluxes) launch_species_integrate(v, species_view(), d_new_cell, stream);  // MxFluxes_Integrate
         mark(4);
         enqueue_scatter(v, b);
@@ -884,14 +1004,14 @@ struct mxg_engine {
             // persistent random forces are redrawn in the first stage only (INTEGRATOR_UPDATE_PERSISTENTFORCE)
             enqueue_singlebody_prep(v, stage == 0);
             if (has_body()) launch_body(v, d_body_f, stream);
-            launch_force(v, has_dpd, force_grid, false, stream);
+            launch_force(v, has_dpd, force_grid, column_split(), false, stream);
             if (has_bonded()) launch_bonded(v, bonded_view(), stream);
             if (stage < 3) {
-                launch_rk_stage(v, d_pos[b], d_rk, stage, !has_bonded(), stream);
+                launch_rk_stage(v, d_pos[b], d_rk, stage, !has_bonded() && needs_combine(), stream);
                 launch_sort_bounds(v, stream);
             } else {
                 launch_rk_final(v, d_pos[b], d_vel[b], d_rk, d_new_cell, d_in_count[b], d_in_list, d_out_count[b],
-                                !has_bonded(), stream);
+                                !has_bonded() && needs_combine(), stream);
             }
         }
         enqueue_scatter(v, b);
@@ -1099,12 +1219,52 @@ int mxg_engine::start(cudaStream_t st) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         num_sms = sms;
     }
+    // The spaces the column force kernel covers have no items here: their columns are its items, a
+    // column's groups of 32 particles shared out over about as many warps as it has groups on
+    // average, and a few to spare (a warp that finds no group ends at once, one that finds several
+    // takes them in turn).
+    std::vector<char> by_column(spaces.size());
+    std::vector<long long> rep_parts(spaces.size(), 0);
+    for (int p : prep) ++rep_parts[p];
+    std::vector<int4> hcol;
+    const bool recorded = records_hold();
+    // The cell kernel evaluates each pair once where the columns do it from both sides, so it keeps the
+    // engines with costly pair terms while its candidates are few: cells of up to 1.2 cutoffs with 11
+    // particles or more, 8 where a DPD term draws from the Philox stream or is summed with a table (below
+    // that it waits for loads). DPD with the reference's random term is cheap enough everywhere. Cells /
+    // columns, step: DPD with Philox, 64,000 cells of 13, edge 1.0: 884 / 1004 us, edge 1.14: 951 / 921; of
+    // 9: 587 / 583; of 6: 374 / 347; of 3: 274 / 181; Morse + DPD, 32,768 in 2,197 cells: 100 / 117; Morse,
+    // 252,000 in 24 boxes, 12 to 16 a cell, edge 1.0 to 1.08: 302 / 300. Force pass: Lennard-Jones, 10 a
+    // cell, edge 1.0: 205 / 176; 20, edge 1.25: 231 / 169.
+    bool any_dpd = false, costly = false;
+    for (const Space &sp : spaces)
+        for (size_t k = 0; k < sp.pot_idx.size(); ++k)
+            for (int q : {sp.pot_idx[k], sp.pot2_idx[k]}) {
+                if (q < 0) continue;
+                any_dpd = any_dpd || pots[q].kind == kKindDPD;
+                costly = costly || pots[q].kind != kKindDPD || (pots[q].flags & kFlagShifted) || q == sp.pot2_idx[k];
+            }
+    costly = !any_dpd || costly || rng_mode != 0;
+    for (size_t r = 0; r < spaces.size(); ++r) {
+        const Space &sp = spaces[r];
+        const bool few_candidates = rep_parts[r] >= (any_dpd ? 8LL : 11LL) * sp.ncells && sp.h[2] < 1.2 * cutoff;
+        by_column[r] = recorded && sp.columns_apply(cutoff) && !(costly && few_candidates);
+        if (!by_column[r]) continue;
+        const int ncol = sp.cdim[0] * sp.cdim[1], cz = sp.cdim[2];
+        const double mean = (double)rep_parts[r] / ncol / 32.0;
+        const int step = std::max(1, (int)std::ceil(1.15 * mean + 0.5));
+        for (int c = 0; c < ncol; ++c)
+            for (int g = 0; g < step; ++g) hcol.push_back(make_int4(sp.cell_offset + c * cz, g, step, cz));
+    }
+    ncol_items = (int)hcol.size();
+    const double mean_groups = (double)(occupancy_hint > 0 ? occupancy_hint : (long long)nparts) / 32.0;
+    col_split = mean_groups >= 8.0 * num_sms ? 1 : mean_groups >= 2.0 * num_sms ? 4 : 8;
     const bool crowded = (occupancy_hint > 0 ? occupancy_hint : (long long)nparts) >= 16LL * std::max(1, ncells);
     const int want_warps = num_sms * (crowded ? 64 : 5 * kWarpsPerBlock);
     const int parts = std::max(1, std::min(kMaxCellParts, (want_warps + ncells - 1) / std::max(1, ncells)));
     std::vector<int> nb_off(ncells + 1, 0), nb_cell, nb_rev, hplanes(ncells, 0);
     std::vector<float4> nb_shift;
-    std::vector<int4> hitems;
+    std::vector<int4> hitems, hall;
     for (int c = 0; c < ncells; ++c) {
         std::vector<const NbEntry *> self_e, first_e, second_e;
         for (auto &e : nb[c]) {
@@ -1118,6 +1278,10 @@ int mxg_engine::start(cudaStream_t st) {
             nb_shift.push_back(e->shift);
             nb_rev.push_back(e->rev);
         };
+        auto put = [&](const int4 &item) {
+            if (!by_column[hrep[c]]) hitems.push_back(item);
+            hall.push_back(item);
+        };
         // a split cell's SELF entry is an item of its own (the crowded cells' n^2 own pairs
         // would otherwise make their first item the longest of the launch)
         const bool self_alone = parts > 1 && !self_e.empty() && nf >= 2;
@@ -1126,20 +1290,21 @@ int mxg_engine::start(cudaStream_t st) {
         if (self_alone) {
             const int e0 = (int)nb_cell.size();
             for (auto *e : self_e) push(e);
-            hitems.push_back(make_int4(c, e0, (int)nb_cell.size(), 0));
+            put(make_int4(c, e0, (int)nb_cell.size(), 0));
         }
         for (int g = 0; g < fgroups; ++g) {
             const int e0 = (int)nb_cell.size();
             if (g == 0 && !self_alone)
                 for (auto *e : self_e) push(e);
             for (int k = g * nf / fgroups; k < (g + 1) * nf / fgroups; ++k) push(first_e[k]);
-            hitems.push_back(make_int4(c, e0, (int)nb_cell.size(), g + (self_alone ? 1 : 0)));
+            put(make_int4(c, e0, (int)nb_cell.size(), g + (self_alone ? 1 : 0)));
         }
         for (auto *e : second_e) push(e);
         nb_off[c + 1] = (int)nb_cell.size();
-        hplanes[c] = hsec[c] + groups - 1;
+        hplanes[c] = by_column[hrep[c]] ? 0 : hsec[c] + groups - 1;
     }
     nitems = (int)hitems.size();
+    nall_items = (int)hall.size();
     h_nb_off = nb_off;
     // few crowded cells, split into several items each: the launch's length is set by the
     // most crowded cells' items, so they are handed out first (reordered before every force
@@ -1206,6 +1371,8 @@ int mxg_engine::start(cudaStream_t st) {
     for (int k : hpidx2)
         if (k >= 0) dpd_pure = false;
     h_pot_idx = hpidx;
+    h_pot_idx2 = hpidx2;
+    const std::vector<float4> hrec = pair_records(hp, hpidx), hrec2 = pair_records(hp, has_second ? hpidx2 : std::vector<int>());
     const std::vector<float4> hdpd = dpd_records(hp);
     has_sb = has_berendsen = has_persist = false;
     has_walls = false;
@@ -1390,6 +1557,8 @@ int mxg_engine::start(cudaStream_t st) {
     rc |= alloc(&d_sec_count, ncells);
     rc |= alloc(&d_cell_planes, ncells);
     rc |= alloc(&d_items, hitems.size());
+    rc |= alloc(&d_col_items, hcol.size());
+    rc |= alloc(&d_all_items, hall.size());
     rc |= alloc(&d_item_ctr, 2);
     rc |= alloc(&d_item_order, hitems.size());
     rc |= alloc(&d_planes, (size_t)nplanes * nparts);
@@ -1398,6 +1567,8 @@ int mxg_engine::start(cudaStream_t st) {
     rc |= alloc(&d_pot_idx, hpidx.size());
     rc |= alloc(&d_pot_idx2, hpidx2.size());
     rc |= alloc(&d_dpd_pair, hdpd.size());
+    rc |= alloc(&d_pair_rec, hrec.size());
+    rc |= alloc(&d_pair_rec2, hrec2.size());
     std::vector<DevCuboid> hcub;
     for (const CuboidInfo &ci : cuboids) {
         DevCuboid d;
@@ -1424,7 +1595,8 @@ int mxg_engine::start(cudaStream_t st) {
     rc |= alloc(&d_spaces, hs.size());
     rc |= alloc(&d_axes, 1);
     rc |= alloc(&d_sort_bounds, (size_t)ncells * 13);
-    rc |= alloc(&d_epot_cell, nitems);
+    rc |= alloc(&d_cell_near, (size_t)ncells);
+    rc |= alloc(&d_epot_cell, (size_t)nitems + kColumnParts * (size_t)ncol_items);
     rc |= alloc(&d_ebond_slot, nparts);
     rc |= alloc(&d_body_e, nparts);
     rc |= alloc(&d_body_f, nparts);
@@ -1470,12 +1642,14 @@ int mxg_engine::start(cudaStream_t st) {
     CUDA_TRY(cudaMemsetAsync(d_status, 0, sizeof(unsigned), stream));
     CUDA_TRY(cudaMemsetAsync(d_step, 0, sizeof(unsigned long long), stream));
     CUDA_TRY(cudaMemsetAsync(d_item_ctr, 0, 2 * sizeof(int), stream));
-    CUDA_TRY(cudaMemsetAsync(d_epot_cell, 0, sizeof(double) * std::max(1, nitems), stream));
+    CUDA_TRY(cudaMemsetAsync(d_epot_cell, 0,
+                             sizeof(double) * std::max<size_t>(1, (size_t)nitems + kColumnParts * (size_t)ncol_items), stream));
     CUDA_TRY(cudaMemsetAsync(d_ebond_slot, 0, sizeof(double) * std::max(1, nparts), stream));
     CUDA_TRY(cudaMemsetAsync(d_body_e, 0, sizeof(double) * std::max(1, nparts), stream));
     if (smax > 0) CUDA_TRY(cudaMemsetAsync(d_rate, 0, sizeof(float) * (size_t)nparts * smax, stream));
     CUDA_TRY(cudaMemsetAsync(d_force, 0, sizeof(float4) * std::max(1, nparts), stream));
     CUDA_TRY(cudaMemsetAsync(d_persist, 0, sizeof(float4) * std::max(1, nparts), stream));
+    CUDA_TRY(cudaMemsetAsync(d_cell_near, 0, sizeof(int) * (size_t)ncells, stream));
     CUDA_TRY(cudaMemsetAsync(d_red_done, 0, 2 * sizeof(unsigned), stream));
     CUDA_TRY(cudaMemsetAsync(d_type_ke, 0, sizeof(double) * ht.size(), stream));
     if ((rc = upload(d_pos[0], hpos, stream)) || (rc = upload(d_vel[0], hvel, stream)) ||
@@ -1485,9 +1659,10 @@ int mxg_engine::start(cudaStream_t st) {
         (rc = upload(d_nb_off, nb_off, stream)) || (rc = upload(d_nb_cell, nb_cell, stream)) ||
         (rc = upload(d_nb_shift, nb_shift, stream)) || (rc = upload(d_nb_rev, nb_rev, stream)) ||
         (rc = upload(d_sec_count, hsec, stream)) || (rc = upload(d_cell_planes, hplanes, stream)) ||
-        (rc = upload(d_items, hitems, stream)) || (rc = upload(d_pots, hp, stream)) ||
+        (rc = upload(d_items, hitems, stream)) || (rc = upload(d_col_items, hcol, stream)) || (rc = upload(d_all_items, hall, stream)) || (rc = upload(d_pots, hp, stream)) ||
         (rc = upload(d_coef, coef, stream)) || (rc = upload(d_pot_idx, hpidx, stream)) ||
         (rc = upload(d_pot_idx2, hpidx2, stream)) || (rc = upload(d_dpd_pair, hdpd, stream)) ||
+        (rc = upload(d_pair_rec, hrec, stream)) || (rc = upload(d_pair_rec2, hrec2, stream)) ||
         (rc = upload(d_cuboids, hcub, stream)) ||
         (rc = upload(d_types, ht, stream)) || (rc = upload(d_spaces, hs, stream)) || (rc = upload(d_axes, haxes, stream)) ||
         (rc = upload(d_bonds, hb, stream)) || (rc = upload(d_bond_flags, hbf, stream)) ||
@@ -1506,7 +1681,11 @@ int mxg_engine::start(cudaStream_t st) {
     CUDA_TRY(cudaStreamSynchronize(stream));
 
     configure_force_kernels();
+    configure_column_kernels();
+    // the cell kernel's warps fetch items, so no more blocks than it needs; the column kernel's blocks
+    // take an item each
     force_grid = std::max(1, std::min((nitems + kWarpsPerBlock - 1) / kWarpsPerBlock, num_sms * 16));
+    force_grid = std::max(force_grid, ncol_items);
     cur = 0;
     started = true;
     refresh_bounds();
@@ -1909,9 +2088,11 @@ int mxg_engine_set_pot_params(mxg_engine *e, int idx, const double *params, int 
     std::vector<DevPot> hp;
     std::vector<float> coef;
     e->pot_arrays(hp, coef);  // same sizes: a frozen-node refit keeps every table's length
-    const std::vector<float4> hdpd = e->dpd_records(hp);
+    const std::vector<float4> hdpd = e->dpd_records(hp), hrec = e->pair_records(hp, e->h_pot_idx),
+                              hrec2 = e->pair_records(hp, e->has_second ? e->h_pot_idx2 : std::vector<int>());
     if ((rc = upload(e->d_pots, hp, e->stream)) || (rc = upload(e->d_coef, coef, e->stream)) ||
-        (rc = upload(e->d_dpd_pair, hdpd, e->stream)))
+        (rc = upload(e->d_dpd_pair, hdpd, e->stream)) || (rc = upload(e->d_pair_rec, hrec, e->stream)) ||
+        (rc = upload(e->d_pair_rec2, hrec2, e->stream)))
         return rc;
     CUDA_TRY(cudaStreamSynchronize(e->stream));  // the host vectors go out of scope
     return MXG_OK;
@@ -2349,7 +2530,7 @@ int mxg_engine_load(mxg_engine *e, int n, const double *x, const float *v) {
 int mxg_engine_energy(mxg_engine *e, double *epot, double *ekin, double *virial9) {
     if (!e) return MXG_ERR_NULL;
     if (!e->started) return MXG_ERR_STATE;
-    launch_energy(e->nitems, e->d_epot_cell, e->nparts, e->has_bonded() ? e->d_ebond_slot : nullptr,
+    launch_energy(e->nitems + kColumnParts * e->ncol_items, e->d_epot_cell, e->nparts, e->has_bonded() ? e->d_ebond_slot : nullptr,
                   e->has_body() ? e->d_body_e : nullptr, e->d_vel[e->cur], e->d_pos[e->cur], e->d_types, e->d_partials, e->energy_blocks, e->d_red_done, e->d_energy,
                   e->stream);
     double out[2];
@@ -2360,15 +2541,16 @@ int mxg_engine_energy(mxg_engine *e, double *epot, double *ekin, double *virial9
     if (virial9) {
         // the pair virial of the current positions: a force pass in the kernel's
         // virial mode, which writes only its per-warp FP64 partials
-        const int nwarps = e->force_grid * kWarpsPerBlock;
+        const int grid = std::min((e->nall_items + kWarpsPerBlock - 1) / kWarpsPerBlock, e->num_sms * 16);
+        const int nwarps = grid * kWarpsPerBlock;
         if (nwarps > e->virial_cap) {
             if (e->alloc(&e->d_virial_partials, (size_t)nwarps * 6) != MXG_OK) return MXG_ERR_MALLOC;
             if (!e->d_virial_out && e->alloc(&e->d_virial_out, 9) != MXG_OK) return MXG_ERR_MALLOC;
             e->virial_cap = nwarps;
         }
-        EngineView v = e->view(e->cur);
+        EngineView v = e->all_cells_view();
         v.virial_partials = e->d_virial_partials;
-        launch_force(v, e->has_dpd, e->force_grid, false, e->stream);
+        launch_force(v, e->has_dpd, grid, 1, false, e->stream);
         launch_virial_reduce(e->d_virial_partials, nwarps, e->d_virial_out, e->stream);
         if (e->has_bonded()) {
             // the bonded terms' share (bonds active after the last pass, exclusions, angles, dihedrals)
@@ -2477,7 +2659,7 @@ int mxg_engine_copy_state(mxg_engine *e, void *host_pos, void *host_vel, int to_
 int mxg_engine_energy_async(mxg_engine *e, double *host_out2) {
     if (!e || !host_out2) return MXG_ERR_NULL;
     if (!e->started) return MXG_ERR_STATE;
-    launch_energy(e->nitems, e->d_epot_cell, e->nparts, e->has_bonded() ? e->d_ebond_slot : nullptr,
+    launch_energy(e->nitems + kColumnParts * e->ncol_items, e->d_epot_cell, e->nparts, e->has_bonded() ? e->d_ebond_slot : nullptr,
                   e->has_body() ? e->d_body_e : nullptr, e->d_vel[e->cur], e->d_pos[e->cur], e->d_types, e->d_partials, e->energy_blocks, e->d_red_done, e->d_energy,
                   e->stream);
     CUDA_TRY(cudaMemcpyAsync(host_out2, e->d_energy, 2 * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
@@ -2582,7 +2764,7 @@ int mxg_engine_vjp_step_forces(mxg_engine *e, void *lam_x, void *lam_v, double *
         CUDA_TRY(cudaMemcpyAsync(e->d_force, forces, sizeof(float4) * (size_t)e->nparts, cudaMemcpyDeviceToDevice,
                                  e->stream));
     else
-        launch_force(v, e->has_dpd, e->force_grid, !bonded, e->stream);
+        launch_force(v, e->has_dpd, e->force_grid, e->column_split(), !bonded, e->stream);
     BondedView bv;
     if (bonded) {
         bv = e->bonded_view();
@@ -2658,7 +2840,7 @@ int mxg_engine_time_force(mxg_engine *e, int reps, double *ms) {
     CUDA_TRY(cudaEventCreate(&b));
     const EngineView v = e->view(e->cur);
     CUDA_TRY(cudaEventRecord(a, e->stream));
-    for (int r = 0; r < reps; ++r) launch_force(v, e->has_dpd, e->force_grid, true, e->stream);
+    for (int r = 0; r < reps; ++r) launch_force(v, e->has_dpd, e->force_grid, e->column_split(), true, e->stream);
     e->force_layout = e->cur;
     CUDA_TRY(cudaEventRecord(b, e->stream));
     CUDA_TRY(cudaEventSynchronize(b));
@@ -2682,7 +2864,7 @@ int mxg_engine_time_force_launches(mxg_engine *e, int reps, void *flush, size_t 
     for (int r = 0; r < reps && err == cudaSuccess; ++r) {
         if (flush_bytes > 0) err = cudaMemsetAsync(flush, 0, flush_bytes, e->stream);
         if (err == cudaSuccess) err = cudaEventRecord(ev[2 * r], e->stream);
-        if (err == cudaSuccess) launch_force(v, e->has_dpd, e->force_grid, false, e->stream);
+        if (err == cudaSuccess) launch_force(v, e->has_dpd, e->force_grid, e->column_split(), false, e->stream);
         if (err == cudaSuccess) err = cudaEventRecord(ev[2 * r + 1], e->stream);
     }
     if (err == cudaSuccess) {
@@ -2708,7 +2890,6 @@ int mxg_engine_autotune(mxg_engine *e) {
     if (!e->started) return MXG_ERR_STATE;
     if (e->nparts == 0) return MXG_OK;
     const int cands[] = {2, 4, 6, 8, 12, 16, 24, 32};
-    const int max_grid = (e->nitems + kWarpsPerBlock - 1) / kWarpsPerBlock;
     int best = e->force_grid, best_per_sm = 0, best_variant = e->force_variant;
     float best_ms = 1e30f;
     cudaEvent_t ev[6];
@@ -2716,13 +2897,14 @@ int mxg_engine_autotune(mxg_engine *e) {
     for (int variant = 0; variant < force_variants(); ++variant) {
         e->force_variant = variant;
         const EngineView v = e->view(e->cur);
+        const int max_grid = e->max_force_grid();
         for (int per_sm : cands) {
             const int grid = std::max(1, std::min(max_grid, e->num_sms * per_sm));
-            launch_force(v, e->has_dpd, grid, true, e->stream);  // warm
+            launch_force(v, e->has_dpd, grid, e->column_split(), true, e->stream);  // warm
             float t[5];
             for (int r = 0; r < 5; ++r) {
                 CUDA_TRY(cudaEventRecord(ev[r], e->stream));
-                launch_force(v, e->has_dpd, grid, true, e->stream);
+                launch_force(v, e->has_dpd, grid, e->column_split(), true, e->stream);
                 CUDA_TRY(cudaEventRecord(ev[5], e->stream));
                 CUDA_TRY(cudaEventSynchronize(ev[5]));
                 cudaEventElapsedTime(&t[r], ev[r], ev[5]);
@@ -2755,8 +2937,8 @@ int mxg_engine_force_config(mxg_engine *e, int *variant, int *grid, int set) {
     if (!e->started) return MXG_ERR_STATE;
     if (*variant < 0 || *variant >= force_variants() || *grid < 1) return MXG_ERR_ARG;
     // no more blocks than the work items can occupy (the autotuner's bound too)
-    *grid = std::min(*grid, std::max(1, (e->nitems + kWarpsPerBlock - 1) / kWarpsPerBlock));
     e->force_variant = *variant;
+    *grid = std::min(*grid, std::max(1, e->max_force_grid()));
     e->force_grid = *grid;
     return e->build_graphs();
 }
@@ -2804,16 +2986,15 @@ int mxg_engine_pair_counts(mxg_engine *e, long long *candidates, long long *inte
         }
     if (candidates) *candidates = cand;
     if (interacting) {
-        // one statistics launch of the force kernel counts the interacting pairs
+        // one statistics launch of the cell kernel counts the interacting pairs
         // (each pair once, in the reference's orientation)
         unsigned long long *d_cnt = nullptr;
         CUDA_TRY(cudaMalloc(&d_cnt, sizeof(unsigned long long)));
         CUDA_TRY(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long), e->stream));
-        EngineView v = e->view(e->cur);
+        EngineView v = e->all_cells_view();
         v.pair_stats = d_cnt;
-        if (e->has_body()) launch_body(v, e->d_body_f, e->stream);
-        launch_force(v, e->has_dpd, e->force_grid, true, e->stream);
-        e->force_layout = e->cur;
+        launch_force(v, e->has_dpd, e->num_sms * 16, 1, false, e->stream);
+        e->enqueue_force(e->cur);  // and the complete forces of the state, as engine_force leaves them
         unsigned long long n = 0;
         CUDA_TRY(cudaMemcpyAsync(&n, d_cnt, sizeof(n), cudaMemcpyDeviceToHost, e->stream));
         CUDA_TRY(cudaStreamSynchronize(e->stream));

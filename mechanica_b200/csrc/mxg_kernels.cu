@@ -16,6 +16,8 @@
  * reference's scalar CPU code bit for bit; only the order of the per-particle
  * force sums differs.
  */
+#include <algorithm>
+
 #include "mxg_device.cuh"
 #include "mxg_kernels.h"
 
@@ -35,11 +37,22 @@ constexpr unsigned kFull = 0xffffffffu;
  * Per cell and per sort direction, the smallest and largest projection key of
  * its particles (runner_dosort.cpp:133-141 computes the keys; runner_dopair
  * reads the largest key of its first cell and the smallest of its second,
- * runner_dopair.cpp:167-171). Called by one warp for one cell.
+ * runner_dopair.cpp:167-171), and whether a particle is within a few key quanta of
+ * a face of the cell (edge h) or outside it: a pair of cells can only be skipped by the
+ * keys' wrap where both cells hold such a particle (within 2 / dscale / |n_k| of the face on
+ * every axis k of the direction n: at most 3.5 quanta). Called by one warp for one cell.
  */
+constexpr int kNearQuanta = 6;
 __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos, int start, int n, float bias,
-                                                 float dscale, const SortAxes *axes, int2 *out) {
+                                                 float dscale, const float *h, int2 *out, int *near_out) {
     const int lane = threadIdx.x & 31;
+    bool near = false;
+    // the axes' directions: 4 along x, 10 along y, 12 along z
+    auto near_face = [&](int sid, int kmin, int kmax) {
+        const int k = sid == 4 ? 0 : sid == 10 ? 1 : 2;
+        near |= kmin <= (int)__fmul_rn(dscale, bias) + kNearQuanta ||
+                kmax >= (int)__fmul_rn(dscale, __fadd_rn(bias, h[k])) - kNearQuanta;
+    };
     if (n <= 32) {  // one particle per lane
         const bool live = lane < n;
         const float4 q = live ? pos[start + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -48,8 +61,10 @@ __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos,
             const int key = sort_key_sid(sid, q.x, q.y, q.z, bias, dscale);
             const int kmin = __reduce_min_sync(kFull, live ? key : 0x7fffffff);
             const int kmax = __reduce_max_sync(kFull, live ? key : -1);
+            if (sid == 4 || sid == 10 || sid == 12) near_face(sid, kmin, kmax);
             if (lane == 0) out[sid] = make_int2(kmin, kmax);
         }
+        if (lane == 0) *near_out = near;
         return;
     }
 #pragma unroll
@@ -63,8 +78,10 @@ __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos,
         }
         kmin = __reduce_min_sync(kFull, kmin);
         kmax = __reduce_max_sync(kFull, kmax);
+        if (sid == 4 || sid == 10 || sid == 12) near_face(sid, kmin, kmax);
         if (lane == 0) out[sid] = make_int2(kmin, kmax);
     }
+    if (lane == 0) *near_out = near;
 }
 
 /* Key bounds of every cell of the current state, for states that did not come
@@ -76,7 +93,7 @@ __global__ void sort_bounds_kernel(EngineView v) {
         if (n == 0) continue;
         const DevSpace &S = v.spaces[v.cell_rep[c]];
         if (!(S.prune & 2)) continue;
-        cell_sort_bounds(v.pos, v.cell_start[c], n, S.sort_bias, S.sort_dscale, v.axes, v.sort_bounds + c * 13);
+        cell_sort_bounds(v.pos, v.cell_start[c], n, S.sort_bias, S.sort_dscale, S.h, v.sort_bounds + c * 13, v.cell_near + c);
     }
 }
 
@@ -578,7 +595,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, TS::kBlocks) force_kernel
         const int n = v.cell_count[c];
         double ecell = 0.0;
         if (n == 0) {
-            for (int e = nb0; e < nb1 && kMode != 2; ++e) {
+            for (int e = nb0; e < nb1 && kMode == 0; ++e) {
                 const int pk = __float_as_int(v.nb_shift[e].w);
                 if ((pk & 3) != kRoleFirst) continue;
                 const int nc = v.nb_cell[e];
@@ -641,7 +658,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, TS::kBlocks) force_kernel
                         }
                     }
                     // skipped pairs owe their neighbour a zero plane (written by the first own chunk)
-                    unsigned zmask = __ballot_sync(kFull, skipped > 0 && i0 == 0 && kMode != 2);
+                    unsigned zmask = __ballot_sync(kFull, skipped > 0 && i0 == 0 && kMode == 0);
                     while (zmask) {
                         const int k = __ffs(zmask) - 1;
                         zmask &= zmask - 1;
@@ -865,7 +882,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, TS::kBlocks) force_kernel
                         __syncwarp();
                         // ---- neighbour-side sums of FIRST entries into their planes; those of a
                         // cell's own particles (pairs evaluated once) into their own sums
-                        for (int idx = lane; idx < M && kMode != 2; idx += 32) {
+                        for (int idx = lane; idx < M && kMode == 0; idx += 32) {
                             const int meta = __float_as_int(sm.nb_s[idx].w);
                             const float4 g0 = sm.nb_f[idx], g1 = sm.nb_f1[idx];
                             const float4 g = make_float4(g0.x + g1.x, g0.y + g1.y, g0.z + g1.z, 0.f);
@@ -894,12 +911,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, TS::kBlocks) force_kernel
                     const float4 f = sm.own_f[k];
                     // the cell's first work item writes the force, later ones their own plane
                     float4 *dst = part == 0 ? v.force : v.planes + (size_t)(v.sec_count[c] + part - 1) * v.nparts;
-                    if (kMode != 2) dst[start + i0 + k] = make_float4(f.x, f.y, f.z, 0.f);
+                    if (kMode == 0) dst[start + i0 + k] = make_float4(f.x, f.y, f.z, 0.f);
                 }
             }
         }
         for (int off = 16; off > 0; off >>= 1) ecell += __shfl_xor_sync(kFull, ecell, off);
-        if (lane == 0 && kMode != 2) v.epot_cell[it] = ecell;
+        if (lane == 0 && kMode == 0) v.epot_cell[it] = ecell;
     }
     if (kMode != 2 && lane == 0) {
         // every warp has drawn its last ticket once the done count reaches the grid's warps:
@@ -2313,7 +2330,7 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 5) scatter_kernel(
         const DevSpace &S = v.spaces[v.cell_rep[c]];
         __syncwarp();
         if (nn > 0 && (S.prune & 2))
-            cell_sort_bounds(pos_out, base, nn, S.sort_bias, S.sort_dscale, v.axes, v.sort_bounds + c * 13);
+            cell_sort_bounds(pos_out, base, nn, S.sort_bias, S.sort_dscale, S.h, v.sort_bounds + c * 13, v.cell_near + c);
     }
     __syncthreads();
     if (tid == 0) {
@@ -2481,7 +2498,7 @@ __global__ void load_order_kernel(EngineView v, LoadView ld, const int *__restri
         }
         __syncwarp();
         const DevSpace &S = v.spaces[v.cell_rep[c]];
-        if (n > 0 && (S.prune & 2)) cell_sort_bounds(pos_out, s0, n, S.sort_bias, S.sort_dscale, v.axes, sort_bounds + c * 13);
+        if (n > 0 && (S.prune & 2)) cell_sort_bounds(pos_out, s0, n, S.sort_bias, S.sort_dscale, S.h, sort_bounds + c * 13, v.cell_near + c);
     }
 }
 
@@ -2699,13 +2716,18 @@ __global__ void item_order_kernel(EngineView v) {
 
 int force_variants() { return kForceVariants; }
 
-void launch_force(const EngineView &v, bool has_dpd, int grid, bool combine, cudaStream_t st) {
-    if (v.item_order && v.nitems > 0 && !v.virial_partials) item_order_kernel<<<1, 1024, 0, st>>>(v);
-    if (has_dpd)
-        launch_force_mode<true>(v, grid, v.force_variant, st);
-    else
-        launch_force_mode<false>(v, grid, v.force_variant, st);
-    if (combine) combine_kernel<<<(v.nparts + 255) / 256, 256, 0, st>>>(v);
+void launch_force(const EngineView &v, bool has_dpd, int grid, int split, bool combine, cudaStream_t st) {
+    launch_column_force(v, has_dpd, split, grid, st);
+    if (v.nitems > 0) {
+        if (v.item_order && !v.virial_partials) item_order_kernel<<<1, 1024, 0, st>>>(v);
+        const int blocks = std::max(1, std::min(grid, (v.nitems + kWarpsPerBlock - 1) / kWarpsPerBlock));
+        if (has_dpd)
+            launch_force_mode<true>(v, blocks, v.force_variant, st);
+        else
+            launch_force_mode<false>(v, blocks, v.force_variant, st);
+    }
+    // the column kernel's forces are complete unless walls, cuboids or single-body forces add to them
+    if (combine && (v.nitems > 0 || v.body_f || v.has_sb)) combine_kernel<<<(v.nparts + 255) / 256, 256, 0, st>>>(v);
 }
 
 int type_ke_blocks(int nparts) { return (nparts + kKeThreads * kKePer - 1) / (kKeThreads * kKePer); }

@@ -25,8 +25,13 @@ void launch_virial_reduce(const double *partials, int nwarps, double *out9, cuda
 int bonded_virial_blocks(int num_sms);
 void launch_bonded_virial(const EngineView &v, const BondedView &bv, int nb, int nx, int na, int nd, int nblocks,
                           double *partials, double *out9, cudaStream_t st);
-/* combine: add the received planes here (no bond or integrator pass follows) */
-void launch_force(const EngineView &v, bool has_dpd, int grid, bool combine, cudaStream_t st);
+/* Forces of the spaces whose cells are cubic and no smaller than the cutoff (mxg_force.cu); split: 1, 4
+ * or 8 warps per group of 32 particles; grid: blocks at most (an item each) */
+constexpr int kColumnParts = 8;     // energy rows per column item: the widest split's warps
+void configure_column_kernels();
+void launch_column_force(const EngineView &v, bool has_dpd, int split, int grid, cudaStream_t st);
+/* combine: add the received planes here (no bond or integrator pass follows); split: as above */
+void launch_force(const EngineView &v, bool has_dpd, int grid, int split, bool combine, cudaStream_t st);
 /* wall and large-particle forces (into body_f) and energies (v.body_e) of the current positions; before
  * the pass's force kernel */
 void launch_body(const EngineView &v, float4 *body_f, cudaStream_t st);
