@@ -145,6 +145,7 @@ struct DevSpace {        // one per replica
     float near_cut;          // relative width in r^2 within which its decisions at a cutoff are left to the
                              // reference's arithmetic
     int off_cell;
+    int flux_columns;        // species fluxes by the column kernel
     double dt_d;         // the engine's dt in double (species integration)
     double cutoff_d;     // the space's cutoff in double (flux weight)
 };

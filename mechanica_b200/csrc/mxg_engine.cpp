@@ -530,6 +530,9 @@ struct mxg_engine {
     int nall_items = 0;
     int4 *d_col_items = nullptr;        // the column force kernel's items
     int ncol_items = 0;
+    int4 *d_flux_items = nullptr;       // the column kernel's items of the species fluxes
+    int nflux_items = 0;
+    bool flux_cells = false;            // some space's fluxes take the per-particle kernel
     int col_split = 1;                  // warps per group of the column force kernel
     DevPot *d_pots = nullptr;
     float *d_coef = nullptr;
@@ -930,7 +933,14 @@ struct mxg_engine {
         if (has_body()) launch_body(v, d_body_f, stream);
         launch_force(v, has_dpd, force_grid, column_split(), !has_bonded(), stream);
         if (has_bonded()) launch_bonded(v, bonded_view(), stream);
-        if (has_fluxes) launch_fluxes(v, species_view(), stream);
+        if (has_fluxes) enqueue_fluxes(v);
+    }
+
+    void enqueue_fluxes(EngineView v) {
+        if (flux_cells) launch_fluxes(v, species_view(), stream);
+        v.col_items = d_flux_items;
+        v.ncol_items = nflux_items;
+        launch_column_fluxes(v, species_view(), column_split(), stream);
     }
 
     SpeciesView species_view() const {
@@ -976,7 +986,7 @@ struct mxg_engine {
         launch_force(v, has_dpd, force_grid, column_split(), false, stream);
         mark(2);
         if (has_bonded()) launch_bonded(v, bonded_view(), stream);
-        if (has_fluxes) launch_fluxes(v, species_view(), stream);
+        if (has_fluxes) enqueue_fluxes(v);
         mark(3);
         launch_integrate(v, d_pos[b], d_vel[b], d_new_cell, d_in_count[b], d_in_list, d_out_count[b],
                          !has_bonded() && needs_combine(), stream);
@@ -1226,7 +1236,9 @@ int mxg_engine::start(cudaStream_t st) {
     std::vector<char> by_column(spaces.size());
     std::vector<long long> rep_parts(spaces.size(), 0);
     for (int p : prep) ++rep_parts[p];
-    std::vector<int4> hcol;
+    std::vector<int4> hcol, hfluxcol;
+    std::vector<char> hflux_columns(spaces.size(), 0);
+    flux_cells = false;
     const bool recorded = records_hold();
     // The cell kernel evaluates each pair once where the columns do it from both sides, so it keeps the
     // engines with costly pair terms while its candidates are few: cells of up to 1.2 cutoffs with 11
@@ -1249,14 +1261,22 @@ int mxg_engine::start(cudaStream_t st) {
         const Space &sp = spaces[r];
         const bool few_candidates = rep_parts[r] >= (any_dpd ? 8LL : 11LL) * sp.ncells && sp.h[2] < 1.2 * cutoff;
         by_column[r] = recorded && sp.columns_apply(cutoff) && !(costly && few_candidates);
-        if (!by_column[r]) continue;
+        const bool flux_columns = has_fluxes && sp.columns_apply(cutoff);
+        hflux_columns[r] = flux_columns;
+        flux_cells = flux_cells || !flux_columns;
+        if (!by_column[r] && !flux_columns) continue;
         const int ncol = sp.cdim[0] * sp.cdim[1], cz = sp.cdim[2];
         const double mean = (double)rep_parts[r] / ncol / 32.0;
         const int step = std::max(1, (int)std::ceil(1.15 * mean + 0.5));
         for (int c = 0; c < ncol; ++c)
-            for (int g = 0; g < step; ++g) hcol.push_back(make_int4(sp.cell_offset + c * cz, g, step, cz));
+            for (int g = 0; g < step; ++g) {
+                const int4 item = make_int4(sp.cell_offset + c * cz, g, step, cz);
+                if (by_column[r]) hcol.push_back(item);
+                if (flux_columns) hfluxcol.push_back(item);
+            }
     }
     ncol_items = (int)hcol.size();
+    nflux_items = (int)hfluxcol.size();
     const double mean_groups = (double)(occupancy_hint > 0 ? occupancy_hint : (long long)nparts) / 32.0;
     col_split = mean_groups >= 8.0 * num_sms ? 1 : mean_groups >= 2.0 * num_sms ? 4 : 8;
     const bool crowded = (occupancy_hint > 0 ? occupancy_hint : (long long)nparts) >= 16LL * std::max(1, ncells);
@@ -1332,6 +1352,7 @@ int mxg_engine::start(cudaStream_t st) {
                 if (p2 >= 0) has_second = true;
             }
         hs.push_back(space_desc(r, r * tt));
+        hs.back().flux_columns = hflux_columns[r];
     }
     // ---- large particles (radius > cutoff: PARTICLE_LARGE, MxParticle.cpp:2091-2093): kept in
     // their cells but static and out of the cell-pair loop; every other particle of the replica
@@ -1559,6 +1580,7 @@ int mxg_engine::start(cudaStream_t st) {
     rc |= alloc(&d_items, hitems.size());
     rc |= alloc(&d_col_items, hcol.size());
     rc |= alloc(&d_all_items, hall.size());
+    rc |= alloc(&d_flux_items, hfluxcol.size());
     rc |= alloc(&d_item_ctr, 2);
     rc |= alloc(&d_item_order, hitems.size());
     rc |= alloc(&d_planes, (size_t)nplanes * nparts);
@@ -1659,7 +1681,7 @@ int mxg_engine::start(cudaStream_t st) {
         (rc = upload(d_nb_off, nb_off, stream)) || (rc = upload(d_nb_cell, nb_cell, stream)) ||
         (rc = upload(d_nb_shift, nb_shift, stream)) || (rc = upload(d_nb_rev, nb_rev, stream)) ||
         (rc = upload(d_sec_count, hsec, stream)) || (rc = upload(d_cell_planes, hplanes, stream)) ||
-        (rc = upload(d_items, hitems, stream)) || (rc = upload(d_col_items, hcol, stream)) || (rc = upload(d_all_items, hall, stream)) || (rc = upload(d_pots, hp, stream)) ||
+        (rc = upload(d_items, hitems, stream)) || (rc = upload(d_col_items, hcol, stream)) || (rc = upload(d_all_items, hall, stream)) || (rc = upload(d_flux_items, hfluxcol, stream)) || (rc = upload(d_pots, hp, stream)) ||
         (rc = upload(d_coef, coef, stream)) || (rc = upload(d_pot_idx, hpidx, stream)) ||
         (rc = upload(d_pot_idx2, hpidx2, stream)) || (rc = upload(d_dpd_pair, hdpd, stream)) ||
         (rc = upload(d_pair_rec, hrec, stream)) || (rc = upload(d_pair_rec2, hrec2, stream)) ||

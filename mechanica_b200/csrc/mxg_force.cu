@@ -48,18 +48,20 @@ constexpr unsigned kFull = 0xffffffffu;
 
 /* What the force terms of an engine can be: tables only; tables, DPD, summed second terms, Philox;
  * DPD only with the reference's random term. */
-enum : int { kTerms = 0, kTermsDpd = 1, kTermsPureDpd = 2 };
+enum : int { kTerms = 0, kTermsDpd = 1, kTermsPureDpd = 2, kTermsFlux = 3 };  // the last: species fluxes, no forces
+__host__ __device__ constexpr bool needs_velocities(int kind) { return kind == kTermsDpd || kind == kTermsPureDpd; }
 
 template <int kKind>
 struct ColSmem {
-    static constexpr int kCap = kKind == kTerms ? 448 : 288;          // staged particles (a multiple of 32)
+    static constexpr int kCap = needs_velocities(kKind) ? 288 : 448;          // staged particles (a multiple of 32)
     int4 nb[kCap + 1];                               // staged position; w = (z + 1) << 11 | code << 6 | type
-    float4 nb_v[kKind == kTerms ? 1 : kCap + 1]; // velocity, w = id
+    float4 nb_v[needs_velocities(kKind) ? kCap + 1 : 1];  // velocity, w = id
     ulonglong2 own_xy[32], own_zr[32];           // candidate test: pairs of -2 x, -2 y, -2 z; widened cutoff^2 - |x|^2
     unsigned mask[kCap / 32 + 1][32];            // neighbours found, per group of 32 staged and own particle
     int4 run[27];                                // runs of slots staged: first slot less offset, end, cell base, code
     int4 off[27];                                // and their shift from the warp's frame, in units
-    int slot[kKind == kTermsPureDpd ? 1 : kCap]; // slot of the staged particle (for odd_pairs)
+    int slot[kKind == kTermsPureDpd ? 1 : kCap]; // slot of the staged particle (for odd_pairs); fluxes: its id
+    float rate[kKind == kTermsFlux ? 8 : 1][32];  // fluxes: the own particles' rates
     int self[32];                                // own particle's staged index in this region, or -1
 };
 
@@ -370,10 +372,44 @@ __device__ __noinline__ ColSums odd_pairs(const EngineView &v, ColSmem<kKind> &s
     return sum;
 }
 
+/* The species fluxes of one pair, seen from the own particle. The kernel's third use: the staging and the
+ * candidates find the pairs, the values are gathered by id. Bound: the latency of those gathers. 50,021
+ * particles of 4 in a cell, 17 neighbours each, five flux entries over three type pairs: 213 us with one
+ * thread a particle walking 27 cells (flux_kernel, kept for other spaces), 66 us here.
+ * flux_eval_ex (flux_eval.hpp:33-84): weight
+ * (1 - r/cutoff)^2 formed in FP64 from the FP32 distance as there, q from the entry's a to its b particle
+ * (the pair's first is a when both types are), decay from both. own_first: in the reference's order. */
+template <int kKind>
+__device__ __forceinline__ void pair_fluxes(const EngineView &v, const SpeciesView &sp, ColSmem<kKind> &sm, int lane, int id,
+                                            int type, int id_j, int type_j, bool own_first, float r, double inv_cutoff) {
+    const int t1 = own_first ? type : type_j, t2 = own_first ? type_j : type;
+    const int f0 = sp.flux_off[t1 * v.ntypes + t2], f1 = sp.flux_off[t1 * v.ntypes + t2 + 1];
+    if (f0 == f1) return;
+    float w = (float)__fma_rn(-(double)r, inv_cutoff, 1.0);
+    w = __fmul_rn(w, w);
+    const int id1 = own_first ? id : id_j, id2 = own_first ? id_j : id;
+    for (int q = f0; q < f1; ++q) {
+        const DevFlux &F = sp.flux[q];
+        const int ida = t1 == F.ta ? id1 : id2, idb = t2 == F.tb ? id2 : id1;
+        const float sa = sp.value[(size_t)ida * sp.smax + F.ia], sb = sp.value[(size_t)idb * sp.smax + F.ib];
+        float g;
+        if (F.kind == 0)
+            g = __fmul_rn(F.k, __fsub_rn(sa, sb));
+        else if (F.kind == 1)
+            g = fmaxf(__fmul_rn(F.k, __fsub_rn(sa, F.target)), 0.f);
+        else
+            g = fmaxf(__fmul_rn(__fmul_rn(F.k, __fsub_rn(F.target, sb)), sa), 0.f);
+        const float qq = __fmul_rn(w, g), hd = __fmul_rn(F.decay, 0.5f);
+        if (ida == id) sm.rate[F.ia][lane] = __fsub_rn(__fsub_rn(sm.rate[F.ia][lane], qq), __fmul_rn(hd, sa));
+        if (idb == id) sm.rate[F.ib][lane] = __fsub_rn(__fadd_rn(sm.rate[F.ib][lane], qq), __fmul_rn(hd, sb));
+    }
+}
+
 /* kSplit warps of a block share a group of particles: each takes every kSplit-th 64 of the particles to
  * be staged, and their sums are added in order. */
 template <int kKind, int kSplit>
-__global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(const __grid_constant__ EngineView v) {
+__global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(const __grid_constant__ EngineView v,
+                                                                              const __grid_constant__ SpeciesView sp) {
     using Smem = ColSmem<kKind>;
     extern __shared__ float4 col_smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -394,6 +430,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             const float4 xi = live ? v.pos[s0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
             ColOwn own;
             own.vel = (kKind != kTerms && live) ? v.vel[s0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const int own_id = __float_as_int(own.vel.w);  // but for tables
             own.type = __float_as_int(xi.w);
             own.slot = s0 + lane;
             const int zi = live ? v.cell_of[s0 + lane] - cell0 : 0;
@@ -494,10 +531,11 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             __syncwarp();
             // with one type the pair's constants stay in registers
             const bool one_type = ntypes == 1;
-            constexpr int kBatch = kKind == kTerms ? 2 : 3;  // rounds of 32 loaded together: more cost registers
+            constexpr int kBatch = needs_velocities(kKind) ? 3 : 2;  // rounds of 32 loaded together: more cost registers
             const int pair_base = S.pot_offset + own.type * ntypes;
             const unsigned rng_mode = S.rng_mode;
             const float wide = 1.f + S.near_cut;
+            const double inv_cutoff = 1.0 / S.cutoff_d;
             float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
             if (kKind == kTermsPureDpd && one_type) {
                 q0 = __ldg(v.dpd_pair + 2 * S.pot_offset);
@@ -505,7 +543,12 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             }
             PairRec rec;
             rec.p = rec.q = q0;
-            if (kKind != kTermsPureDpd && one_type) rec = load_rec(v.pair_rec, S.pot_offset);
+            if (kKind == kTermsFlux) {
+                const bool first = live && w == 0;  // the carried rates, once
+                for (int k = 0; k < 8; ++k)
+                    sm.rate[k][lane] = first && k < sp.smax ? sp.rate[(size_t)own_id * sp.smax + k] : 0.f;
+            }
+            if ((kKind == kTerms || kKind == kTermsDpd) && one_type) rec = load_rec(v.pair_rec, S.pot_offset);
             float3 f = make_float3(0.f, 0.f, 0.f);
             // this warp's rounds: of every 64 particles the 32 with even places, then, from the start again,
             // those with odd ones. The halves are alike in space, so when a region holds one of them a
@@ -561,18 +604,19 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                         if (keep) {
                             const int at = base + __popc(bal & lt_mask);
                             sm.nb[at] = b;
-                            if (kKind != kTerms) cp_async16(&sm.nb_v[at], v.vel + slot[r]);
-                            if (kKind != kTermsPureDpd) sm.slot[at] = slot[r];
+                            if (needs_velocities(kKind)) cp_async16(&sm.nb_v[at], v.vel + slot[r]);
+                            if (kKind != kTermsPureDpd)
+                                sm.slot[at] = kKind == kTermsFlux ? __float_as_int(v.vel[slot[r]].w) : slot[r];
                             if (cq[r] == 4 && (unsigned)(slot[r] - s0) < (unsigned)nown) sm.self[slot[r] - s0] = at;
                         }
                         base += __popc(bal);
                     }
                 }
-                if (kKind != kTerms) cp_async_wait_all();
+                if (needs_velocities(kKind)) cp_async_wait_all();
                 if (lane == 0) {  // the place past the last
                     const int far = 0x40000000;
                     sm.nb[Smem::kCap] = make_int4(far, far, far, 0);
-                    if (kKind != kTerms) sm.nb_v[Smem::kCap] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (needs_velocities(kKind)) sm.nb_v[Smem::kCap] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
                 __syncwarp();
                 // ---- candidates
@@ -622,8 +666,18 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                     const float dx = (float)(own.x - b.x), dy = (float)(own.y - b.y), dz = (float)(own.z - b.z);
                     const float s2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));  // r^2 in units^2
                     const bool within = s2 <= cut2;
-                    float fs, tx = dx, ty = dy, tz = dz;
-                    if (kKind == kTermsPureDpd) {
+                    float fs = 0.f, tx = dx, ty = dy, tz = dz;
+                    if constexpr (kKind == kTermsFlux) {
+                        // the weight vanishes at the cutoff: which side a pair within a rounding of it takes is moot
+                        if (!within) return;
+                        const float r = fminf(__fsqrt_rn(s2) * unit, (float)S.cutoff_d);
+                        const int c9 = ((b.w >> 6) & 31) % 9;
+                        const int side = (c9 / 3 - 1) * 9 + (c9 % 3 - 1) * 3 + (b.w >> 11) - 1 - own.zrel;
+                        const int id_j = sm.slot[jj];  // in a cell the lower slot is first, the lower id too
+                        pair_fluxes<kKind>(v, sp, sm, lane, own_id, own.type, id_j, b.w & 63, side > 0 || (side == 0 && own_id < id_j),
+                                           r, inv_cutoff);
+                        return;
+                    } else if constexpr (kKind == kTermsPureDpd) {
                         if (!one_type) {
                             const int pk = pair_base + (b.w & 63);
                             q0 = __ldg(v.dpd_pair + 2 * pk);
@@ -681,7 +735,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                     pair(ja);
                     pair(jb);
                 }
-                if (__any_sync(kFull, odd)) {
+                if (kKind != kTermsFlux && __any_sync(kFull, odd)) {
                     const ColSums c = odd_pairs<kKind>(v, sm, S, own, loc[0], loc[1], zi, unit, ngrp, live);
                     sum.x += c.x;
                     sum.y += c.y;
@@ -693,6 +747,19 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                 f.z += sum.z;
                 energy += sum.e;
                 __syncwarp();
+            }
+            if constexpr (kKind == kTermsFlux) {
+                __syncwarp();
+                if (kSplit > 1) __syncthreads();
+                if (live && w == 0 && sp.nspec[own.type] > 0) {
+                    for (int k = 0; k < sp.smax; ++k) {
+                        float t = sm.rate[k][lane];
+                        for (int q = 1; q < kSplit; ++q) t += reinterpret_cast<Smem *>(col_smem)[q].rate[k][lane];
+                        sp.rate[(size_t)own_id * sp.smax + k] = t;
+                    }
+                }
+                if (kSplit > 1) __syncthreads();
+                continue;
             }
             if (kSplit > 1) {  // the warps' sums, in order
                 float4 *share = reinterpret_cast<float4 *>(sm.own_xy);
@@ -719,7 +786,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
         }
         // ---- the item's energy (DPD tabulates none): every pair was met from both sides. A row for each
         // warp of the widest split
-        if (kKind != kTermsPureDpd) {
+        if (kKind == kTerms || kKind == kTermsDpd) {
             double e = 0.5 * energy;
             for (int off = 16; off > 0; off >>= 1) e += __shfl_xor_sync(kFull, e, off);
             double *row = v.epot_cell + v.nitems + kColumnParts * it;
@@ -738,19 +805,19 @@ void configure_one() {
 }
 
 template <int kKind, int kSplit>
-void launch_one(const EngineView &v, int grid, cudaStream_t st) {
+void launch_one(const EngineView &v, const SpeciesView &sp, int grid, cudaStream_t st) {
     const int blocks = std::max(1, std::min(grid, v.ncol_items));
-    column_force_kernel<kKind, kSplit><<<blocks, 32 * kSplit, sizeof(ColSmem<kKind>) * kSplit, st>>>(v);
+    column_force_kernel<kKind, kSplit><<<blocks, 32 * kSplit, sizeof(ColSmem<kKind>) * kSplit, st>>>(v, sp);
 }
 
 template <int kKind>
-void launch_kind(const EngineView &v, int split, int grid, cudaStream_t st) {
+void launch_kind(const EngineView &v, const SpeciesView &sp, int split, int grid, cudaStream_t st) {
     if (split >= 8)
-        launch_one<kKind, 8>(v, grid, st);
+        launch_one<kKind, 8>(v, sp, grid, st);
     else if (split >= 4)
-        launch_one<kKind, 4>(v, grid, st);
+        launch_one<kKind, 4>(v, sp, grid, st);
     else
-        launch_one<kKind, 1>(v, grid, st);
+        launch_one<kKind, 1>(v, sp, grid, st);
 }
 
 template <int kKind>
@@ -766,16 +833,22 @@ void configure_column_kernels() {
     configure_kind<kTerms>();
     configure_kind<kTermsDpd>();
     configure_kind<kTermsPureDpd>();
+    configure_kind<kTermsFlux>();
+}
+
+void launch_column_fluxes(const EngineView &v, const SpeciesView &sp, int split, cudaStream_t st) {
+    if (v.ncol_items > 0) launch_kind<kTermsFlux>(v, sp, split, v.ncol_items, st);
 }
 
 void launch_column_force(const EngineView &v, bool has_dpd, int split, int grid, cudaStream_t st) {
     if (v.ncol_items == 0) return;
+    const SpeciesView none{};
     if (has_dpd && v.dpd_pure)
-        launch_kind<kTermsPureDpd>(v, split, grid, st);
+        launch_kind<kTermsPureDpd>(v, none, split, grid, st);
     else if (has_dpd || v.pot_idx2)
-        launch_kind<kTermsDpd>(v, split, grid, st);
+        launch_kind<kTermsDpd>(v, none, split, grid, st);
     else
-        launch_kind<kTerms>(v, split, grid, st);
+        launch_kind<kTerms>(v, none, split, grid, st);
 }
 
 }  // namespace mxg

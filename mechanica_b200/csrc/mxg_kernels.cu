@@ -1069,6 +1069,7 @@ __global__ void flux_kernel(EngineView v, SpeciesView sp) {
     for (int k = 0; k < 8; ++k) acc[k] = k < sp.smax ? rate[k] : 0.f;
     const int c = v.cell_of[s];
     const DevSpace &S = v.spaces[v.cell_rep[c]];
+    if (S.flux_columns) return;
     const bool exit_test = (S.prune & 2) != 0;
     for (int e = sp.fx_off[c]; e < sp.fx_off[c + 1]; ++e) {
         const int nc = sp.fx_cell[e];

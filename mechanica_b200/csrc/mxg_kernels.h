@@ -30,12 +30,15 @@ void launch_bonded_virial(const EngineView &v, const BondedView &bv, int nb, int
 constexpr int kColumnParts = 8;     // energy rows per column item: the widest split's warps
 void configure_column_kernels();
 void launch_column_force(const EngineView &v, bool has_dpd, int split, int grid, cudaStream_t st);
+/* Species fluxes of the spaces with DevSpace::flux_columns; v.col_items: their columns */
+void launch_column_fluxes(const EngineView &v, const SpeciesView &sp, int split, cudaStream_t st);
 /* combine: add the received planes here (no bond or integrator pass follows); split: as above */
 void launch_force(const EngineView &v, bool has_dpd, int grid, int split, bool combine, cudaStream_t st);
 /* wall and large-particle forces (into body_f) and energies (v.body_e) of the current positions; before
  * the pass's force kernel */
 void launch_body(const EngineView &v, float4 *body_f, cudaStream_t st);
-/* species flux rates of the current positions (full shell, by particle id), added to the carried rates */
+/* species flux rates of the current positions (full shell, by particle id), added to the carried rates, of
+ * the spaces without DevSpace::flux_columns */
 void launch_fluxes(const EngineView &v, const SpeciesView &sp, cudaStream_t st);
 /* species values += dt * rates after a forward-Euler step for particles that kept their cell (new_cell
  * from the integrator); v is the state the rates belong to */
