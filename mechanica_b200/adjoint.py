@@ -56,11 +56,14 @@ class Parameters:
 
     def apply(self, theta):
         theta = np.asarray(theta, dtype=np.float64)
+        new = {}  # a potential with several parameters is re-fitted once
         for k, entries in enumerate(self.slots):
             for pot, j in entries:
-                q = self.construction(pot)
-                q[j] = theta[k]
-                self.u.set_potential_params(pot, q)
+                if pot not in new:
+                    new[pot] = self.construction(pot)
+                new[pot][j] = theta[k]
+        for pot, q in new.items():
+            self.u.set_potential_params(pot, q)
 
     def register(self):
         """Tells the engine which (engine potential, parameter) feeds which slot: every
