@@ -262,7 +262,8 @@ struct EngineView {      // everything a kernel needs, passed by value
     const int4 *items;       // force work items: (cell, first entry, end entry, part)
     int *item_ctr;           // [0] next work item, [1] warps done (dynamic fetch; zero between launches)
     int *item_order;         // items by decreasing cell occupancy (split cells only), else null
-    int dpd_pure;            // every pair potential is DPD with the reference's random term: DPD-only kernel
+    int dpd_pure;            // every pair potential is DPD (not shifted): DPD-only kernel; 1: the reference's
+                             // random term, 2: the Philox stream
     int force_variant;       // the force kernel's tile shape (see Tile), chosen by the autotuner
     int nitems;
     const DevCuboid *cuboids;  // static cuboids (all replicas)

@@ -523,7 +523,7 @@ struct mxg_engine {
     int *d_item_order = nullptr;        // work items, most crowded cells first (when cells are split)
     bool order_items = false;
     long long occupancy_hint = 0;       // particle count the work-item split is decided on (0: nparts)
-    bool dpd_pure = false;              // every pair potential DPD, no summed second term, no Philox
+    bool dpd_pure = false;              // every pair potential DPD (not shifted), no summed second term
     int *d_cell_planes = nullptr;       // planes summed into each cell's forces
     int nitems = 0;
     int4 *d_all_items = nullptr;        // the cell kernel's items with every cell (pair counts and virial)
@@ -869,7 +869,7 @@ struct mxg_engine {
         v.items = d_items;
         v.item_ctr = d_item_ctr;
         v.item_order = order_items ? d_item_order : nullptr;
-        v.dpd_pure = dpd_pure ? 1 : 0;
+        v.dpd_pure = !dpd_pure ? 0 : rng_mode == 0 ? 1 : 2;
         v.force_variant = force_variant;
         v.nitems = nitems;
         v.col_items = d_col_items;
@@ -1386,7 +1386,7 @@ int mxg_engine::start(cudaStream_t st) {
                 hpidx[k] = -1;  // large particles take no part in the cell-pair loop
                 hpidx2[k] = -1;
             }
-    dpd_pure = has_dpd && rng_mode == 0;
+    dpd_pure = has_dpd;
     for (int k : hpidx)
         if (k >= 0 && (pots[k].kind != kKindDPD || (pots[k].flags & kFlagShifted))) dpd_pure = false;
     for (int k : hpidx2)

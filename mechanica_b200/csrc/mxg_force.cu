@@ -124,17 +124,22 @@ __device__ __forceinline__ bool pair_term(const EngineView &v, const PairRec &re
     e = 0.f;
     if (kKind != kTerms && rec.code() < 0) {
         if (r2 > __fmul_rn(rec.p.y, rec.p.y) || rec.code() == -2) return false;
-        const float ir = rsqrt_ftz(r2);
-        const float sr = __fmaf_rn(r2, ir, -rec.p.w);
-        const float oc = sr < 0.f ? 1.f : __fmaf_rn(-sr, rec.p.z, 1.0f);
+        // r, 1/r and the quotient by the cutoff one Newton step on from the unit's results: as close to
+        // the FP64 values as divisions (DPD mixed with tables, shifted, or with the Philox stream)
+        float ir = rsqrt_ftz(r2);
+        float r = __fmul_rn(r2, ir);
+        r = __fmaf_rn(__fmaf_rn(-r, r, r2), 0.5f * ir, r);
+        ir = __fmaf_rn(__fmaf_rn(-r, ir, 1.0f), ir, ir);
+        const float sr = __fsub_rn(r, rec.p.w), qt = __fmul_rn(sr, rec.p.z);
+        const float oc = sr < 0.f ? 1.f : __fmaf_rn(__fmaf_rn(qt, rec.p.y, -sr), rec.p.z, __fsub_rn(1.0f, qt));
         const float dv = __fmaf_rn(dx, __fsub_rn(vi.x, vj.x),
                                    __fmaf_rn(dy, __fsub_rn(vi.y, vj.y), __fmul_rn(dz, __fsub_rn(vi.z, vj.z))));
-        float rnd = rec.q.z;
+        float xi = 1.f;
         if (rng_mode) {
             const unsigned idi = __float_as_uint(vi.w), idj = __float_as_uint(vj.w);
-            rnd = __fmul_rn(rnd, philox_pair_xi(*v.step, min(idi, idj), max(idi, idj)));
+            xi = philox_pair_xi(*v.step, min(idi, idj), max(idi, idj));
         }
-        fs = dpd_term(oc, ir, dv, rec.q.y, __fadd_rn(rec.q.x, rnd));
+        fs = dpd_term(oc, ir, dv, rec.q.y, __fmaf_rn(rec.q.z, xi, rec.q.x));
         return true;
     }
     if (!table_term(rec, v.coef, r2, e, fs)) return false;
@@ -843,7 +848,7 @@ void launch_column_fluxes(const EngineView &v, const SpeciesView &sp, int split,
 void launch_column_force(const EngineView &v, bool has_dpd, int split, int grid, cudaStream_t st) {
     if (v.ncol_items == 0) return;
     const SpeciesView none{};
-    if (has_dpd && v.dpd_pure)
+    if (has_dpd && v.dpd_pure == 1)
         launch_kind<kTermsPureDpd>(v, none, split, grid, st);
     else if (has_dpd || v.pot_idx2)
         launch_kind<kTermsDpd>(v, none, split, grid, st);
