@@ -22,7 +22,6 @@ namespace mxg {
 constexpr int kChunk = 8;           // floats per table interval
 constexpr int kBucket = 32;         // movers per cell per step kept in the cell's bucket (more go to the overflow list)
 constexpr int kChunkShift = 8;      // the re-binning's net mover counts per chunk of 256 consecutive cells
-constexpr int kScatterWarps = 8;    // re-binning: cells (one warp each) per block
 constexpr int kMaxTypes = 64;       // types per engine
 constexpr int kWarpsPerBlock = 4;   // force kernel: warps (work items) per block
 constexpr int kMaxCellParts = 8;    // force work items per cell at most
@@ -305,9 +304,14 @@ __device__ __forceinline__ uint4 philox4x32(uint4 c, uint2 k) {
 
 /* The reference's projection key of a particle along sort direction n
  * (runner_dosort.cpp:133-136): (unsigned)(dscale * (bias + x.n)) in FP32. */
-__device__ __forceinline__ int sort_key(float x, float y, float z, const float *n, float bias, float dscale) {
-    const float proj = __fadd_rn(__fadd_rn(__fadd_rn(bias, __fmul_rn(x, n[0])), __fmul_rn(y, n[1])), __fmul_rn(z, n[2]));
+__device__ __forceinline__ float sort_projection(float x, float y, float z, const float *n, float bias) {
+    return __fadd_rn(__fadd_rn(__fadd_rn(bias, __fmul_rn(x, n[0])), __fmul_rn(y, n[1])), __fmul_rn(z, n[2]));
+}
+__device__ __forceinline__ int projection_key(float proj, float dscale) {
     return (int)(unsigned)__fmul_rn(dscale, proj);
+}
+__device__ __forceinline__ int sort_key(float x, float y, float z, const float *n, float bias, float dscale) {
+    return projection_key(sort_projection(x, y, z, n, bias), dscale);
 }
 
 /* sort_key along the reference's sort direction sid (runner_dosort.cpp's 13 normalised cell
@@ -332,6 +336,14 @@ __device__ __forceinline__ int sort_key_sid(int sid, float x, float y, float z, 
         default: n[0] = 0.f; n[1] = 0.f; n[2] = 1.f; break;
     }
     return sort_key(x, y, z, n, bias, dscale);
+}
+
+/* The sort direction sid as a vector, the same values. */
+__device__ __forceinline__ void sort_axis(int sid, float n[3]) {
+    const int o[3] = {sid < 9 ? 1 : 0, 1 - (sid / 3) % 3, 1 - sid % 3};
+    const int k = abs(o[0]) + abs(o[1]) + abs(o[2]);
+    const float a = k == 3 ? (float)5.773502691896258e-01 : k == 2 ? (float)7.071067811865475e-01 : 1.f;
+    for (int d = 0; d < 3; ++d) n[d] = (float)o[d] * a;
 }
 
 /* Cell coordinates of global cell c in its replica's grid. */

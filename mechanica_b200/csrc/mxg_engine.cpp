@@ -1001,7 +1001,7 @@ struct mxg_engine {
         launch_scatter(v, d_pos[b], d_vel[b], d_new_cell, d_cell_start[b], d_cell_count[b], d_in_count[b], d_in_list,
                        d_out_count[b], d_cell_start[nb], d_cell_count[nb], d_pos[nb], d_vel[nb], d_cell_of[nb],
                        d_slot_of_id, d_in_count[nb], d_out_count[nb], d_chunk_delta[nb], nchunks, d_rebin_ctl,
-                       d_step, stream);
+                       d_step, num_sms, stream);
     }
 
     /* One Runge-Kutta 4 step (engine_advance_runge_kutta_4): four force passes (with

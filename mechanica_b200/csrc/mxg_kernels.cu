@@ -43,16 +43,17 @@ constexpr unsigned kFull = 0xffffffffu;
  * every axis k of the direction n: at most 3.5 quanta). Called by one warp for one cell.
  */
 constexpr int kNearQuanta = 6;
-__device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos, int start, int n, float bias,
-                                                 float dscale, const float *h, int2 *out, int *near_out) {
+__device__ __forceinline__ int axis_sid(int k) { return k == 0 ? 4 : k == 1 ? 10 : 12; }  // the axes' directions
+__device__ __forceinline__ bool near_face(const DevSpace &S, int k, int kmin, int kmax) {
+    return kmin <= (int)__fmul_rn(S.sort_dscale, S.sort_bias) + kNearQuanta ||
+           kmax >= (int)__fmul_rn(S.sort_dscale, __fadd_rn(S.sort_bias, S.h[k])) - kNearQuanta;
+}
+
+__device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos, int start, int n, const DevSpace &S,
+                                                 int2 *out, int *near_out) {
     const int lane = threadIdx.x & 31;
+    const float bias = S.sort_bias, dscale = S.sort_dscale;
     bool near = false;
-    // the axes' directions: 4 along x, 10 along y, 12 along z
-    auto near_face = [&](int sid, int kmin, int kmax) {
-        const int k = sid == 4 ? 0 : sid == 10 ? 1 : 2;
-        near |= kmin <= (int)__fmul_rn(dscale, bias) + kNearQuanta ||
-                kmax >= (int)__fmul_rn(dscale, __fadd_rn(bias, h[k])) - kNearQuanta;
-    };
     if (n <= 32) {  // one particle per lane
         const bool live = lane < n;
         const float4 q = live ? pos[start + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -61,7 +62,8 @@ __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos,
             const int key = sort_key_sid(sid, q.x, q.y, q.z, bias, dscale);
             const int kmin = __reduce_min_sync(kFull, live ? key : 0x7fffffff);
             const int kmax = __reduce_max_sync(kFull, live ? key : -1);
-            if (sid == 4 || sid == 10 || sid == 12) near_face(sid, kmin, kmax);
+            for (int k = 0; k < 3; ++k)
+                if (sid == axis_sid(k)) near |= near_face(S, k, kmin, kmax);
             if (lane == 0) out[sid] = make_int2(kmin, kmax);
         }
         if (lane == 0) *near_out = near;
@@ -78,7 +80,8 @@ __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos,
         }
         kmin = __reduce_min_sync(kFull, kmin);
         kmax = __reduce_max_sync(kFull, kmax);
-        if (sid == 4 || sid == 10 || sid == 12) near_face(sid, kmin, kmax);
+        for (int k = 0; k < 3; ++k)
+            if (sid == axis_sid(k)) near |= near_face(S, k, kmin, kmax);
         if (lane == 0) out[sid] = make_int2(kmin, kmax);
     }
     if (lane == 0) *near_out = near;
@@ -93,7 +96,7 @@ __global__ void sort_bounds_kernel(EngineView v) {
         if (n == 0) continue;
         const DevSpace &S = v.spaces[v.cell_rep[c]];
         if (!(S.prune & 2)) continue;
-        cell_sort_bounds(v.pos, v.cell_start[c], n, S.sort_bias, S.sort_dscale, S.h, v.sort_bounds + c * 13, v.cell_near + c);
+        cell_sort_bounds(v.pos, v.cell_start[c], n, S, v.sort_bounds + c * 13, v.cell_near + c);
     }
 }
 
@@ -2229,126 +2232,225 @@ __global__ void __launch_bounds__(kAdvThreads, 4) rk_final_kernel(EngineView v, 
 }
 
 /*
- * The stable re-binning into the other buffer: one warp per destination cell, kScatterWarps
- * consecutive cells per block. The cell's new start needs no scan over all cells: it is its
- * old start plus the net number of movers into the cells before it, which the block sums from
- * the integrator's per-chunk net counts (chunks before the block's own) and the per-cell
- * counts of its chunk before its first cell; the block's cells then add up their new counts
- * in order. Stayers keep their relative order (ascending id); movers from the cell's bucket
- * and from the overflow list are merged in by id, so every cell stays sorted by id and the
- * layout does not depend on thread scheduling. The warp then computes the new cell's
- * projection-key bounds for the next force pass.
+ * The stable re-binning into the other buffer: a block per group of consecutive cells, a thread
+ * per particle of the block's contiguous run of slots (the copies are whole lines, and no lane is
+ * idle where cells hold fewer than 32). The group's new start needs no scan over all cells: it is
+ * its old start plus the net number of movers into the cells before it, which the block sums from
+ * the integrator's per-chunk net counts (chunks before the block's own) and the per-cell counts of
+ * its chunk before its first cell; one warp scans the group's new counts. Stayers keep their
+ * relative order (ascending id): their places come from a running count of stayers over the
+ * block's slots. Movers from the cell's bucket and from the overflow list are merged in by id, so
+ * every cell stays sorted by id and the layout does not depend on thread scheduling. Then the new
+ * cells' projection-key bounds for the next force pass, from the positions staged on the way: a
+ * lane per sort direction, 16 lanes a cell, each over the cell's particles.
  *
  * The counts of this step are read by other blocks and stay as they are; the block clears its
  * cells' counts of the other buffer parity (and the grid that parity's chunk counts), which the
  * next step uses. The block that finishes last re-arms its done counter and the overflow list
  * and advances the step counter that keys the Philox streams.
  */
-__global__ void __launch_bounds__(kScatterWarps * 32, 5) scatter_kernel(
-    EngineView v, int ncells, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
+constexpr int kScatterLog2 = 5, kScatterCells = 1 << kScatterLog2;  // most cells of a block
+constexpr int kScatterSlots = 512;   // mean slots of a block at most
+
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 1280 / kThreads) scatter_kernel(
+    EngineView v, int ncells, int group_log2, const float4 *__restrict__ pos, const float4 *__restrict__ vel,
     const int *__restrict__ new_cell, const int *__restrict__ old_start, const int *__restrict__ old_count,
     const int *__restrict__ in_count, const int *__restrict__ in_list, const int *__restrict__ out_count,
     int *new_start, int *new_count, float4 *pos_out, float4 *vel_out, int *cell_out, int *slot_of_id,
     int *clear_in, int *clear_out, int *clear_chunk, int nchunks, unsigned *done, unsigned long long *step) {
-    __shared__ int s_net[kScatterWarps], s_n[kScatterWarps];
+    constexpr int kWarps = kThreads / 32, kRow = kBucket + 1;
+    constexpr int kStage = 4 * kThreads;           // slots whose ids and positions are kept in shared memory
+    __shared__ float4 s_pos[kStage];        // the new slots' positions
+    __shared__ int s_id[kStage];            // the old slots' ids, INT_MAX where the particle leaves
+    __shared__ int s_mover[kScatterCells * kRow];  // ids of the buckets' movers
+    __shared__ int s_kmin[kScatterCells * 13], s_kmax[kScatterCells * 13];
+    __shared__ int s_start[kScatterCells], s_base[kScatterCells + 1], s_first[kScatterCells], s_in[kScatterCells];
+    __shared__ int s_rep[kScatterCells], s_net[kWarps], s_stay[2][kWarps];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int c0 = blockIdx.x * kScatterWarps, c = c0 + wid;
+    const int c0 = blockIdx.x << group_log2, nc = min(1 << group_log2, ncells - c0);
+    const int beg = old_start[c0], end = old_start[c0 + nc - 1] + old_count[c0 + nc - 1];
+
+    // the first slots' particles; later tiles are loaded below
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), u = x;
+    int c = -1, dest = -2;
+    auto load = [&](int s) {
+        c = -1;
+        dest = -2;
+        if (s < end) {
+            x = pos[s];
+            u = vel[s];
+            c = v.cell_of[s];
+            dest = new_cell[s];
+        }
+    };
+    load(beg + tid);
+
+    int nn = 0;  // the first warp's lanes: the new count of a cell
+    if (tid < nc) {
+        const int in = in_count[c0 + tid], on = old_count[c0 + tid];
+        nn = on - out_count[c0 + tid] + in;
+        s_start[tid] = old_start[c0 + tid];
+        s_in[tid] = in;
+        s_rep[tid] = v.cell_rep[c0 + tid];
+        clear_in[c0 + tid] = 0;
+        clear_out[c0 + tid] = 0;
+    }
+    for (int j = blockIdx.x * blockDim.x + tid; j < nchunks; j += gridDim.x * blockDim.x) clear_chunk[j] = 0;
     {
         // net movers into the cells [0, c0): whole chunks, then the cells of c0's chunk before c0
-        const int k0 = c0 >> kChunkShift, cb = k0 << kChunkShift;
+        const int k0 = c0 >> kChunkShift;
         int net = 0;
-        for (int j = tid; j < k0; j += blockDim.x) net += v.chunk_delta[j];
-        for (int q = cb + 4 * tid; q < c0; q += 4 * blockDim.x) {  // [cb, c0) holds whole int4 groups
-            const int4 a = *reinterpret_cast<const int4 *>(in_count + q);
-            const int4 b = *reinterpret_cast<const int4 *>(out_count + q);
-            net += ((a.x + a.y) + (a.z + a.w)) - ((b.x + b.y) + (b.z + b.w));
-        }
+        for (int q = (k0 << kChunkShift) + tid; q < c0; q += kThreads) net += in_count[q] - out_count[q];
+        for (int j = tid; j < k0; j += kThreads) net += v.chunk_delta[j];
         net = __reduce_add_sync(kFull, net);
-        if (lane == 0) {
-            s_net[wid] = net;
-            s_n[wid] = c < ncells ? old_count[c] - out_count[c] + in_count[c] : 0;
-        }
-        for (int j = blockIdx.x * blockDim.x + tid; j < nchunks; j += gridDim.x * blockDim.x) clear_chunk[j] = 0;
-        __syncthreads();
+        if (lane == 0) s_net[wid] = net;
     }
-    if (c < ncells) {
-        int base = old_start[c0];
-        for (int w = 0; w < kScatterWarps; ++w) base += s_net[w] + (w < wid ? s_n[w] : 0);
-        const int os = old_start[c], on = old_count[c];
-        const int mtot = in_count[c];
-        const int m = min(mtot, kBucket);
-        const int nov = mtot > kBucket ? *v.ovf_count : 0;  // the overflow list is scanned only when needed
-        // movers into c with an id below myid: from the bucket, then from the overflow list
-        auto movers_below = [&](int myid) {
-            int r = 0;
-            for (int q = 0; q < m; ++q) r += __float_as_int(vel[in_list[c * kBucket + q]].w) < myid;
+    for (int w = wid; w < nc; w += kWarps)
+        if (lane < min(in_count[c0 + w], kBucket))
+            s_mover[w * kRow + lane] = __float_as_int(vel[in_list[(c0 + w) * kBucket + lane]].w);
+    for (int t = tid; t < nc * 13; t += kThreads) {
+        s_kmin[t] = 0x7fffffff;
+        s_kmax[t] = -1;
+    }
+
+    // movers into cell l of the group with an id below myid: from the bucket, then from the overflow list
+    auto movers_below = [&](int l, int myid) {
+        const int in = s_in[l];
+        int r = 0;
+        for (int q = 0; q < min(in, kBucket); ++q) r += s_mover[l * kRow + q] < myid;
+        if (in > kBucket) {
+            const int nov = *v.ovf_count;
             for (int q = 0; q < nov; ++q) {
                 const int src = v.ovf_list[q];
-                r += new_cell[src] == c && __float_as_int(vel[src].w) < myid;
-            }
-            return r;
-        };
-        auto stayers_below = [&](int myid) {
-            int r = 0;
-            for (int k = 0; k < on; ++k) r += (new_cell[os + k] == c) && (__float_as_int(vel[os + k].w) < myid);
-            return r;
-        };
-        auto place = [&](int src, int myid, int dst) {
-            pos_out[dst] = pos[src];
-            vel_out[dst] = vel[src];
-            cell_out[dst] = c;
-            slot_of_id[myid] = dst;
-        };
-        // stayers
-        int stay_before = 0;
-        for (int k0 = 0; k0 < on; k0 += 32) {
-            const int k = k0 + lane;
-            bool stay = false;
-            int myid = 0;
-            if (k < on) {
-                stay = new_cell[os + k] == c;
-                myid = __float_as_int(vel[os + k].w);
-            }
-            const unsigned bal = __ballot_sync(kFull, stay);
-            if (stay) place(os + k, myid, base + stay_before + __popc(bal & ((1u << lane) - 1u)) + movers_below(myid));
-            stay_before += __popc(bal);
-        }
-        // movers of the bucket
-        for (int q0 = 0; q0 < m; q0 += 32) {
-            const int q = q0 + lane;
-            if (q < m) {
-                const int src = in_list[c * kBucket + q];
-                const int myid = __float_as_int(vel[src].w);
-                place(src, myid, base + stayers_below(myid) + movers_below(myid));
+                r += new_cell[src] == c0 + l && __float_as_int(vel[src].w) < myid;
             }
         }
-        // movers of the overflow list
-        for (int q0 = 0; q0 < nov; q0 += 32) {
-            const int q = q0 + lane;
-            if (q < nov) {
-                const int src = v.ovf_list[q];
-                if (new_cell[src] == c) {
-                    const int myid = __float_as_int(vel[src].w);
-                    place(src, myid, base + stayers_below(myid) + movers_below(myid));
-                }
+        return r;
+    };
+    auto place = [&](int l, const float4 &xs, const float4 &us, int dst) {
+        pos_out[dst] = xs;
+        vel_out[dst] = us;
+        cell_out[dst] = c0 + l;
+        slot_of_id[__float_as_int(us.w)] = dst;
+        if (dst - s_base[0] < kStage) s_pos[dst - s_base[0]] = xs;
+    };
+
+    // stayers, a tile of slots at a time; before: stayers of the block's slots before this one
+    int run = 0, odd = 0;
+    for (int t0 = beg; t0 == beg || t0 < end; t0 += kThreads, odd ^= 1) {
+        const int s = t0 + tid;
+        if (t0 != beg) load(s);
+        const bool stay = dest == c;
+        if (s < end && s - beg < kStage) s_id[s - beg] = stay ? __float_as_int(u.w) : 0x7fffffff;
+        const unsigned bal = __ballot_sync(kFull, stay);
+        if (lane == 0) s_stay[odd][wid] = __popc(bal);
+        __syncthreads();
+        if (t0 == beg && wid == 0) {
+            int incl = nn;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_up_sync(kFull, incl, d);
+                if (lane >= d) incl += o;
+            }
+            const int base = beg + __reduce_add_sync(kFull, lane < kWarps ? s_net[lane] : 0) + incl - nn;
+            if (lane < nc) {
+                s_base[lane] = base;
+                new_start[c0 + lane] = base;
+                new_count[c0 + lane] = nn;
+            }
+            if (lane == nc - 1) {
+                s_base[nc] = base + nn;
+                if (c0 + nc == ncells) new_start[ncells] = base + nn;
             }
         }
-        const int nn = stay_before + mtot;
-        if (lane == 0) {
-            new_start[c] = base;
-            new_count[c] = nn;
-            if (c == ncells - 1) new_start[ncells] = base + nn;
-            clear_in[c] = 0;
-            clear_out[c] = 0;
+        int before = run + __popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const int k = s_stay[odd][w];
+            before += w < wid ? k : 0;
+            run += k;
         }
-        // the next force pass's cell-pair exit test reads the new cell's key bounds from the slots
-        // just written (the barrier makes the lanes' stores visible to the whole warp)
-        const DevSpace &S = v.spaces[v.cell_rep[c]];
-        __syncwarp();
-        if (nn > 0 && (S.prune & 2))
-            cell_sort_bounds(pos_out, base, nn, S.sort_bias, S.sort_dscale, S.h, v.sort_bounds + c * 13, v.cell_near + c);
+        const int l = c - c0;
+        if (s < end && s == s_start[l]) s_first[l] = before;
+        __syncthreads();
+        if (stay) place(l, x, u, s_base[l] + before - s_first[l] + movers_below(l, __float_as_int(u.w)));
+    }
+
+    // movers
+    auto stayers_below = [&](int l, int myid) {
+        const int os = s_start[l], on = old_count[c0 + l];
+        int r = 0;
+        if (os + on - beg <= kStage) {
+            for (int k = 0; k < on; ++k) r += s_id[os - beg + k] < myid;
+        } else {
+            for (int k = 0; k < on; ++k) r += new_cell[os + k] == c0 + l && __float_as_int(vel[os + k].w) < myid;
+        }
+        return r;
+    };
+    for (int w = wid; w < nc; w += kWarps) {
+        if (lane >= min(s_in[w], kBucket)) continue;
+        const int src = in_list[(c0 + w) * kBucket + lane];
+        const float4 xs = pos[src], us = vel[src];
+        const int myid = __float_as_int(us.w);
+        place(w, xs, us, s_base[w] + stayers_below(w, myid) + movers_below(w, myid));
+    }
+    if (__syncthreads_or(tid < nc && s_in[tid] > kBucket)) {  // movers of the overflow list
+        const int nov = *v.ovf_count;
+        for (int q = tid; q < nov; q += kThreads) {
+            const int src = v.ovf_list[q], l = new_cell[src] - c0;
+            if (l < 0 || l >= nc) continue;
+            const float4 us = vel[src];
+            const int myid = __float_as_int(us.w);
+            place(l, pos[src], us, s_base[l] + stayers_below(l, myid) + movers_below(l, myid));
+        }
+        __syncthreads();
+    }
+
+    // the next force pass's cell-pair exit test: the new cells' key bounds, particles dealt to the
+    // 16-lane groups of a cell in turn
+    {
+        const int sid = tid & 15, g = tid >> 4;
+        constexpr int kGroups = kThreads / 16;
+        const int parts_log2 = max(0, 31 - __clz(kGroups) - group_log2), parts = 1 << parts_log2;
+        float n[3];
+        sort_axis(min(sid, 12), n);
+        for (int i = g; i < nc << parts_log2; i += kGroups) {
+            const int l = i >> parts_log2;
+            const int b = s_base[l], e = s_base[l + 1];
+            const DevSpace &S = v.spaces[s_rep[l]];
+            if (!(S.prune & 2)) continue;
+            const float bias = S.sort_bias, dscale = S.sort_dscale;
+            // the key does not fall as the projection rises: one conversion a bound
+            float lo = INFINITY, hi = -INFINITY;
+            auto add = [&](const float4 &q) {
+                const float proj = sort_projection(q.x, q.y, q.z, n, bias);
+                lo = fminf(lo, proj);
+                hi = fmaxf(hi, proj);
+            };
+            const int first = b + (i & (parts - 1)), b0 = s_base[0];
+            if (first >= e) continue;
+            if (e - b0 <= kStage)
+#pragma unroll 2
+                for (int d = first; d < e; d += parts) add(s_pos[d - b0]);
+            else
+                for (int d = first; d < e; d += parts) add(pos_out[d]);
+            const int kmin = projection_key(lo, dscale), kmax = projection_key(hi, dscale);
+            if (sid < 13) {
+                atomicMin(&s_kmin[l * 13 + sid], kmin);
+                atomicMax(&s_kmax[l * 13 + sid], kmax);
+            }
+        }
     }
     __syncthreads();
+    for (int t = tid; t < nc * 13; t += kThreads)
+        if (s_base[t / 13 + 1] > s_base[t / 13]) v.sort_bounds[c0 * 13 + t] = make_int2(s_kmin[t], s_kmax[t]);
+    if (tid < nc && s_base[tid + 1] > s_base[tid] && (v.spaces[s_rep[tid]].prune & 2)) {
+        const DevSpace &S = v.spaces[s_rep[tid]];
+        bool near = false;
+        for (int k = 0; k < 3; ++k) near |= near_face(S, k, s_kmin[tid * 13 + axis_sid(k)], s_kmax[tid * 13 + axis_sid(k)]);
+        v.cell_near[c0 + tid] = near;
+    }
     if (tid == 0) {
         __threadfence();
         if (atomicAdd(done, 1u) == gridDim.x - 1) {  // every block is done with the overflow list
@@ -2514,7 +2616,7 @@ __global__ void load_order_kernel(EngineView v, LoadView ld, const int *__restri
         }
         __syncwarp();
         const DevSpace &S = v.spaces[v.cell_rep[c]];
-        if (n > 0 && (S.prune & 2)) cell_sort_bounds(pos_out, s0, n, S.sort_bias, S.sort_dscale, S.h, sort_bounds + c * 13, v.cell_near + c);
+        if (n > 0 && (S.prune & 2)) cell_sort_bounds(pos_out, s0, n, S, sort_bounds + c * 13, v.cell_near + c);
     }
 }
 
@@ -2815,12 +2917,24 @@ void launch_scatter(const EngineView &v, const float4 *pos, const float4 *vel, c
                     const int *old_start, const int *old_count, const int *in_count, const int *in_list,
                     const int *out_count, int *new_start, int *new_count, float4 *pos_out, float4 *vel_out,
                     int *cell_out, int *slot_of_id, int *clear_in, int *clear_out, int *clear_chunk, int nchunks,
-                    unsigned *ctl, unsigned long long *step, cudaStream_t st) {
-    const int grid = (v.ncells + kScatterWarps - 1) / kScatterWarps;
-    scatter_kernel<<<grid, kScatterWarps * 32, 0, st>>>(v, v.ncells, pos, vel, new_cell, old_start, old_count,
-                                                        in_count, in_list, out_count, new_start, new_count, pos_out,
-                                                        vel_out, cell_out, slot_of_id, clear_in, clear_out,
-                                                        clear_chunk, nchunks, ctl, step);
+                    unsigned *ctl, unsigned long long *step, int sms, cudaStream_t st) {
+    // As many cells a block as give it some 400 particles and every SM two blocks. Blocks of 128 threads wait
+    // less at their barriers but hold a longer run each: from eight blocks an SM up (1,200,007 particles of 11 in a
+    // cell: 58 us, 66 with 256 threads), below that 256 (200,000 of 12.5: 16.5 us, 21 with 128; 10,000 in 4^3 cells:
+    // 9.9, 11.4). A warp a cell took 143, 25 and 22.6 us: idle lanes, a serial chain of loads a cell, 13 single
+    // stores of bounds.
+    int k = kScatterLog2;
+    while (k > 0 && (((long long)v.nparts << k) > (long long)kScatterSlots * v.ncells || v.ncells < (2 * sms) << k)) --k;
+    const int grid = (v.ncells + (1 << k) - 1) >> k;
+    auto launch = [&](auto *kernel, int threads) {
+        kernel<<<grid, threads, 0, st>>>(v, v.ncells, k, pos, vel, new_cell, old_start, old_count, in_count, in_list,
+                                         out_count, new_start, new_count, pos_out, vel_out, cell_out, slot_of_id,
+                                         clear_in, clear_out, clear_chunk, nchunks, ctl, step);
+    };
+    if (grid >= 8 * sms)
+        launch(scatter_kernel<128>, 128);
+    else
+        launch(scatter_kernel<256>, 256);
 }
 
 void launch_number_density(const EngineView &v, const int *flux_off, float *nd_by_id, cudaStream_t st) {

@@ -63,7 +63,7 @@ void launch_scatter(const EngineView &v, const float4 *pos, const float4 *vel, c
                     const int *old_start, const int *old_count, const int *in_count, const int *in_list,
                     const int *out_count, int *new_start, int *new_count, float4 *pos_out, float4 *vel_out,
                     int *cell_out, int *slot_of_id, int *clear_in, int *clear_out, int *clear_chunk, int nchunks,
-                    unsigned *ctl, unsigned long long *step, cudaStream_t st);
+                    unsigned *ctl, unsigned long long *step, int sms, cudaStream_t st);
 /* The particles' number density (f[3] of the reference's particles) for the current positions, by id;
  * flux_off: the species flux lists per type pair (null when there are none). */
 void launch_number_density(const EngineView &v, const int *flux_off, float *nd_by_id, cudaStream_t st);
