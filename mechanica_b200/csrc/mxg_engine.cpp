@@ -932,7 +932,7 @@ struct mxg_engine {
         enqueue_singlebody_prep(v, false);
         if (has_body()) launch_body(v, d_body_f, stream);
         launch_force(v, has_dpd, force_grid, column_split(), !has_bonded(), stream);
-        if (has_bonded()) launch_bonded(v, bonded_view(), stream);
+        if (has_bonded()) launch_bonded(v, bonded_view(), num_sms, stream);
         if (has_fluxes) enqueue_fluxes(v);
     }
 
@@ -985,7 +985,7 @@ struct mxg_engine {
         mark(1);
         launch_force(v, has_dpd, force_grid, column_split(), false, stream);
         mark(2);
-        if (has_bonded()) launch_bonded(v, bonded_view(), stream);
+        if (has_bonded()) launch_bonded(v, bonded_view(), num_sms, stream);
         if (has_fluxes) enqueue_fluxes(v);
         mark(3);
         launch_integrate(v, d_pos[b], d_vel[b], d_new_cell, d_in_count[b], d_in_list, d_out_count[b],
@@ -1015,7 +1015,7 @@ struct mxg_engine {
             enqueue_singlebody_prep(v, stage == 0);
             if (has_body()) launch_body(v, d_body_f, stream);
             launch_force(v, has_dpd, force_grid, column_split(), false, stream);
-            if (has_bonded()) launch_bonded(v, bonded_view(), stream);
+            if (has_bonded()) launch_bonded(v, bonded_view(), num_sms, stream);
             if (stage < 3) {
                 launch_rk_stage(v, d_pos[b], d_rk, stage, !has_bonded() && needs_combine(), stream);
                 launch_sort_bounds(v, stream);
@@ -2790,7 +2790,7 @@ int mxg_engine_vjp_step_forces(mxg_engine *e, void *lam_x, void *lam_v, double *
     BondedView bv;
     if (bonded) {
         bv = e->bonded_view();
-        launch_bonded(v, bv, e->stream);
+        launch_bonded(v, bv, e->num_sms, e->stream);
     }
     e->force_layout = e->cur;
     AdjointView a;

@@ -44,7 +44,7 @@ void launch_fluxes(const EngineView &v, const SpeciesView &sp, cudaStream_t st);
  * from the integrator); v is the state the rates belong to */
 void launch_species_integrate(const EngineView &v, const SpeciesView &sp, const int *new_cell, cudaStream_t st);
 /* bonds then angles; also adds the received planes (the force pass ran without combine) */
-void launch_bonded(const EngineView &v, const BondedView &bv, cudaStream_t st);
+void launch_bonded(const EngineView &v, const BondedView &bv, int sms, cudaStream_t st);
 /* Forward Euler, walls and relocation: movers into the destination's bucket or the overflow list,
  * counted per cell (in_count, out_count) and, between chunks of cells, in v.chunk_delta. */
 void launch_integrate(const EngineView &v, float4 *pos, float4 *vel, int *new_cell, int *in_count, int *in_list,
