@@ -239,6 +239,7 @@ struct EngineView {      // everything a kernel needs, passed by value
     const unsigned long long *step;  // device step counter
     const SortAxes *axes;
     int2 *sort_bounds;               // per cell and sort axis: (min key, max key)
+    const int *slot_of_id;
     int *cell_near;                  // per cell: a particle near a face, by the axes' keys (cell_sort_bounds)
     double *epot_cell;       // per force work item, then kColumnParts per column item: energy of the last force pass
     unsigned *status;

@@ -856,6 +856,7 @@ struct mxg_engine {
         v.axes = d_axes;
         v.sort_bounds = d_sort_bounds;
         v.cell_near = d_cell_near;
+        v.slot_of_id = d_slot_of_id;
         v.epot_cell = d_epot_cell;
         v.status = d_status;
         v.pair_stats = nullptr;

@@ -314,14 +314,42 @@ struct ColOwn {
     float4 vel;
 };
 
+/* The displacement from the particle at slot_j to the one at slot_i as the reference rounds it, d =
+ * (x_first - s) - x_second from the cell-relative positions; side orders the two cells (0: the same cell,
+ * > 0: that of slot_i is the first), c9 and oz are the other cell's place among the nine columns and
+ * along z, (x, y, z) the own cell. */
+__device__ __forceinline__ float3 reference_d(const EngineView &v, const DevSpace &S, int slot_i, int slot_j, int x, int y,
+                                              int z, int c9, int oz, int side) {
+    const float4 xi = v.pos[slot_i], xj = v.pos[slot_j];
+    float s[3] = {0.f, 0.f, 0.f};
+    if (side != 0) neighbour_cell(S, x, y, z, c9 / 3 - 1, c9 % 3 - 1, oz, s);
+    return side < 0 ? make_float3(__fsub_rn(xi.x, __fadd_rn(xj.x, s[0])), __fsub_rn(xi.y, __fadd_rn(xj.y, s[1])),
+                                  __fsub_rn(xi.z, __fadd_rn(xj.z, s[2])))
+                    : make_float3(__fsub_rn(__fsub_rn(xi.x, s[0]), xj.x), __fsub_rn(__fsub_rn(xi.y, s[1]), xj.y),
+                                  __fsub_rn(__fsub_rn(xi.z, s[2]), xj.z));
+}
+
+/* Whether the reference counts a pair near the cutoff as within it (its cell loop's cutoff for pairs of
+ * one cell, its pair loop's for others). */
+__device__ __noinline__ bool reference_within(const EngineView &v, const DevSpace &S, int slot_i, int slot_j, int x, int y,
+                                              int z, int c9, int oz, int side) {
+    const float3 d = reference_d(v, S, slot_i, slot_j, x, y, z, c9, oz, side);
+    return dot3_rn(d.x, d.y, d.z) <= (side == 0 ? S.cut2_self : S.cut2_pair);
+}
+
+/* Closer than 1/64 of the cutoff (r^2 as a fraction of its square), the last bit of a position turns a
+ * pair's direction by 4e-6 and more: such pairs, one particle in 5,000 at twelve in a cell, take the
+ * reference's displacement too. */
+constexpr float kClose2 = 1.0f / 4096.0f;
+
 /* The pairs that the main walk leaves out: those closer than their potential's a, which get a random
- * direction of that length, and those so near to a or to the cutoff that the decision depends on
- * rounding. The reference's arithmetic decides (d = (x_first - s) - x_second from the cell-relative
- * positions, r^2 unfused); a DPD-only pass, whose force vanishes at the cutoff, keeps its own. The main
- * walk clears a lane's bits as it takes them and sets these again; rare, so a walk of its own. */
+ * direction of that length, those so near to a or to the cutoff that the decision depends on rounding
+ * (in a DPD-only pass the force vanishes at the cutoff, and only a counts), and those closer than
+ * kClose2. They take the reference's displacement, r^2 unfused. The main walk clears a lane's bits as it
+ * takes them and sets these again; rare, so a walk of its own. */
 template <int kKind>
 __device__ __noinline__ ColSums odd_pairs(const EngineView &v, ColSmem<kKind> &sm, const DevSpace &S, ColOwn o, int x, int y,
-                                          int z, float unit, int ngroups, bool live) {
+                                          int z, int ngroups, bool live) {
     const int lane = threadIdx.x & 31;
     ColSums sum = {0.f, 0.f, 0.f, 0.0};
     for (int u = 0; u < ngroups; ++u) {
@@ -333,20 +361,11 @@ __device__ __noinline__ ColSums odd_pairs(const EngineView &v, ColSmem<kKind> &s
             const int pk = S.pot_offset + o.type * v.ntypes + (b.w & 63);
             const PairRec rec = load_rec(v.pair_rec, pk);
             if (rec.code() == -2) continue;
-            float3 d = make_float3((float)(o.x - b.x) * unit, (float)(o.y - b.y) * unit, (float)(o.z - b.z) * unit);
-            float cut2 = S.cut2_pair;
-            if (kKind != kTermsPureDpd) {
-                const float4 xi = v.pos[o.slot], xj = v.pos[sm.slot[jj]];
-                const int c9 = ((b.w >> 6) & 31) % 9, oz = (b.w >> 11) - 1 - o.zrel;
-                const int side = (c9 / 3 - 1) * 9 + (c9 % 3 - 1) * 3 + oz;  // 0: own cell, > 0: the first of the two
-                float s[3] = {0.f, 0.f, 0.f};
-                if (side != 0) neighbour_cell(S, x, y, z, c9 / 3 - 1, c9 % 3 - 1, oz, s);
-                if (side == 0) cut2 = S.cut2_self;
-                d = side < 0 ? make_float3(__fsub_rn(xi.x, __fadd_rn(xj.x, s[0])), __fsub_rn(xi.y, __fadd_rn(xj.y, s[1])),
-                                           __fsub_rn(xi.z, __fadd_rn(xj.z, s[2])))
-                             : make_float3(__fsub_rn(__fsub_rn(xi.x, s[0]), xj.x), __fsub_rn(__fsub_rn(xi.y, s[1]), xj.y),
-                                           __fsub_rn(__fsub_rn(xi.z, s[2]), xj.z));
-            }
+            const int slot_j = kKind == kTermsPureDpd ? v.slot_of_id[__float_as_int(sm.nb_v[jj].w)] : sm.slot[jj];
+            const int c9 = ((b.w >> 6) & 31) % 9, oz = (b.w >> 11) - 1 - o.zrel;
+            const int side = (c9 / 3 - 1) * 9 + (c9 % 3 - 1) * 3 + oz;  // 0: own cell, > 0: the first of the two
+            const float cut2 = side == 0 ? S.cut2_self : S.cut2_pair;
+            const float3 d = reference_d(v, S, o.slot, slot_j, x, y, z, c9, oz, side);
             const float r2 = dot3_rn(d.x, d.y, d.z);
             if (r2 > cut2) continue;
             const float4 vj = kKind != kTerms ? sm.nb_v[jj] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -539,7 +558,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             constexpr int kBatch = needs_velocities(kKind) ? 3 : 2;  // rounds of 32 loaded together: more cost registers
             const int pair_base = S.pot_offset + own.type * ntypes;
             const unsigned rng_mode = S.rng_mode;
-            const float wide = 1.f + S.near_cut;
+            const float wide = 1.f + S.near_cut, close2 = kClose2 * S.cut2_pair;
             const double inv_cutoff = 1.0 / S.cutoff_d;
             float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
             if (kKind == kTermsPureDpd && one_type) {
@@ -673,12 +692,15 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                     const bool within = s2 <= cut2;
                     float fs = 0.f, tx = dx, ty = dy, tz = dz;
                     if constexpr (kKind == kTermsFlux) {
-                        // the weight vanishes at the cutoff: which side a pair within a rounding of it takes is moot
                         if (!within) return;
                         const float r = fminf(__fsqrt_rn(s2) * unit, (float)S.cutoff_d);
                         const int c9 = ((b.w >> 6) & 31) % 9;
                         const int side = (c9 / 3 - 1) * 9 + (c9 % 3 - 1) * 3 + (b.w >> 11) - 1 - own.zrel;
                         const int id_j = sm.slot[jj];  // in a cell the lower slot is first, the lower id too
+                        // the weight vanishes at the cutoff, a flux's decay does not
+                        if (s2 > cut2_in && !reference_within(v, S, own.slot, v.slot_of_id[id_j], loc[0], loc[1], zi, c9,
+                                                              (b.w >> 11) - 1 - own.zrel, side))
+                            return;
                         pair_fluxes<kKind>(v, sp, sm, lane, own_id, own.type, id_j, b.w & 63, side > 0 || (side == 0 && own_id < id_j),
                                            r, inv_cutoff);
                         return;
@@ -694,14 +716,14 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                         const float oc = fmaxf(__fmaf_rn(-__fmul_rn(s2, ir), q1.z * unit, 1.0f), 0.f);
                         const float dv = __fmaf_rn(dx, own.vel.x - vj.x, __fmaf_rn(dy, own.vel.y - vj.y, dz * (own.vel.z - vj.z)));
                         fs = dpd_term(oc, ir, dv, q0.z, q1.w);
-                        const bool near = s2 < q1.x * (scale * scale);  // closer than a
+                        const bool near = s2 < fmaxf(q1.x, close2) * (scale * scale);  // than a, or for the direction
                         if (near && within) later(jj);
                         fs = within && !near ? fs : 0.f;
                     } else {
                         const int pk = pair_base + (b.w & 63);
                         if (!one_type) rec = load_rec(v.pair_rec, pk);
                         const float r2 = s2 * (unit * unit);
-                        const bool use = s2 <= cut2_in && r2 >= rec.p.x * wide;
+                        const bool use = s2 <= cut2_in && r2 >= fmaxf(rec.p.x * wide, close2);
                         float e;
                         bool in;
                         tx = dx * unit;
@@ -741,7 +763,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                     pair(jb);
                 }
                 if (kKind != kTermsFlux && __any_sync(kFull, odd)) {
-                    const ColSums c = odd_pairs<kKind>(v, sm, S, own, loc[0], loc[1], zi, unit, ngrp, live);
+                    const ColSums c = odd_pairs<kKind>(v, sm, S, own, loc[0], loc[1], zi, ngrp, live);
                     sum.x += c.x;
                     sum.y += c.y;
                     sum.z += c.z;
