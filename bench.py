@@ -426,7 +426,7 @@ def force_roofline(L, e, flush, f_int, what, reps=20):
     flops = F_CAND * cand.value + f_int * inter.value
     peak, src = fp32_peak_tflops()
     achieved = flops / (ms / 1e3) / 1e12
-    return {"bound": "fp32", "kernel": f"force_kernel ({what})", "achieved": achieved, "peak": peak,
+    return {"bound": "fp32", "kernel": f"force pass ({what})", "achieved": achieved, "peak": peak,
             "unit": "TFLOP/s", "frac": achieved / peak, "peak_source": src, "force_ms_per_launch": ms,
             "algorithmic_flops_per_launch": flops, "candidate_pairs": cand.value, "interacting_pairs": inter.value,
             "flops_per_pair": {"candidate": F_CAND, "interacting": f_int}}
@@ -718,7 +718,7 @@ def main():
     max_mhz = (peaks or {}).get("sm_max_mhz", 1965.0)
     fp32_peak = sm_count * 128 * 2 * max_mhz * 1e6 / 1e12  # TFLOP/s, nominal (no measured FP32 figure)
     achieved = flops / (force_ms / 1e3) / 1e12
-    roofline = {"bound": "fp32", "kernel": "force_kernel (nonbonded cell-pair forces)", "achieved": achieved,
+    roofline = {"bound": "fp32", "kernel": "column_force_kernel (nonbonded forces by columns of cells)", "achieved": achieved,
                 "peak": fp32_peak, "unit": "TFLOP/s", "frac": achieved / fp32_peak,
                 "peak_source": f"nominal FP32 pipe: {sm_count} SMs x 128 lanes x 2 x {max_mhz:.0f} MHz "
                                "(MEASURED_PEAKS.json holds no FP32 figure)",
@@ -755,8 +755,8 @@ def main():
 
     # ---- re-binning against the measured HBM bandwidth: the integrator (advance + mover counts)
     # and the scatter (re-binning + next key bounds), each timed with CUDA events at the phase
-    # boundaries of whole steps (kernel by kernel, no L2 flush: the integrator reads the received
-    # planes the force pass just wrote); algorithmic bytes 88 per particle for each (integrate:
+    # boundaries of whole steps (kernel by kernel, no L2 flush: the integrator reads the forces
+    # the force pass just wrote); algorithmic bytes 88 per particle for each (integrate:
     # pos, vel, force, type read, pos, vel, cell written; scatter: key, pos, vel, id, type read
     # and written) ----
     tm = (ctypes.c_double * 16)()

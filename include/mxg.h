@@ -200,14 +200,15 @@ int mxg_engine_pot_index(mxg_engine *e, int replica, int type_i, int type_j, int
  * engine the device copy is updated in place, ordered on the engine stream. No counterpart in the
  * reference. */
 int mxg_engine_set_pot_params(mxg_engine *e, int idx, const double *params, int nparams);
-/* Chooses the force kernel's tile shape (own and neighbour particles staged per region: 32/96,
- * 32/64, 64/96 or 32/128) and grid (CTAs per SM) by timing candidate launches on the current state,
- * so the choice follows the state's density; returns the chosen blocks per SM. Call after
- * mxg_engine_start. Tile shapes differ in the order of the FP32 force sums, so two engines compare
- * bit for bit only with the same configuration (mxg_engine_force_config). No counterpart in the
- * reference. */
+/* Chooses the force kernels' variant and the grid (CTAs per SM) by timing candidate launches on the
+ * current state, so the choice follows the state's density; returns the chosen blocks per SM. Call
+ * after mxg_engine_start. A variant is, for the cell kernel, the tile shape (own and neighbour
+ * particles staged per region: 32/96, 32/64, 64/96 or 32/128) and, for spaces on the column kernel,
+ * the warps that share 32 particles (0: by the number of groups, 1 to 3: 1, 4 or 8). Variants differ
+ * in the order of the FP32 force sums, so two engines compare bit for bit only with the same
+ * configuration (mxg_engine_force_config). No counterpart in the reference. */
 int mxg_engine_autotune(mxg_engine *e);
-/* set = 0: reads the force kernel's tile variant (0-3) and grid (CTAs); set = 1: pins them (after
+/* set = 0: reads the force kernels' variant (0-3) and grid (CTAs); set = 1: pins them (after
  * mxg_engine_start; the grid is clamped to the blocks the work items can occupy and written back;
  * the step graphs are re-captured). */
 int mxg_engine_force_config(mxg_engine *e, int *variant, int *grid, int set);

@@ -1185,13 +1185,13 @@ class _Universe:
         return ms.value
 
     def autotune(self):
-        """Picks the force kernel's tile shape and grid by timing candidates on the current
+        """Picks the force kernels' variant and grid by timing candidates on the current
         state; returns the chosen CTAs per SM (force_config() gives the variant and grid)."""
         self._ensure()
         return check(lib().mxg_engine_autotune(self._e), "autotune")
 
     def force_config(self, variant=None, grid=None):
-        """(tile variant, grid) of the force kernel; with both arguments, pins them."""
+        """(variant, grid) of the force kernels; with both arguments, pins them."""
         self._ensure()
         vv, gg = ctypes.c_int(0 if variant is None else int(variant)), ctypes.c_int(0 if grid is None else int(grid))
         setting = variant is not None and grid is not None

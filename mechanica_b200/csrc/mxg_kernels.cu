@@ -2,12 +2,14 @@
  * Force-and-step kernels for sm_100a.
  *
  *   force_kernel      nonbonded cell-pair forces (tables, DPD), single-body
- *                     forces, per-cell FP64 energy. One warp per cell.
- *   bonded_kernel     harmonic/table bonds with dissociation flags, angles.
+ *                     forces, per-cell FP64 energy. One warp per cell. (Spaces
+ *                     of columns take the column kernel, mxg_force.cu.)
+ *   bonded_kernel     exclusions, bonds with dissociation flags, angles,
+ *                     dihedrals; one or four lanes per particle.
  *   integrate_kernel  forward Euler (Newtonian / overdamped), speed clamp,
  *                     wall reflection, relocation; counts the next binning.
- *   scatter_kernel    stable re-binning (ascending id inside each cell); each
- *                     cell's new start from chunked net mover counts.
+ *   scatter_kernel    stable re-binning (ascending id inside each cell), a thread
+ *                     per slot; new starts from chunked net mover counts.
  *   energy kernels    FP64 reductions of potential and kinetic energy.
  *
  * Compiled with -fmad=false: every FP32/FP64 operation on the pair, bond and
