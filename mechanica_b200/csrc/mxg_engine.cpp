@@ -1242,13 +1242,15 @@ int mxg_engine::start(cudaStream_t st) {
     flux_cells = false;
     const bool recorded = records_hold();
     // The cell kernel evaluates each pair once where the columns do it from both sides, so it keeps the
-    // engines with costly pair terms while its candidates are few: cells of up to 1.2 cutoffs with 11
+    // engines with costly pair terms while its candidates are few: cells of up to 1.34 cutoffs with 11
     // particles or more, 8 where a DPD term draws from the Philox stream or is summed with a table (below
     // that it waits for loads). DPD with the reference's random term is cheap enough everywhere. Cells /
     // columns, step: DPD with Philox, 64,000 cells of 13, edge 1.0: 884 / 1004 us, edge 1.14: 951 / 921; of
     // 9: 587 / 583; of 6: 374 / 347; of 3: 274 / 181; Morse + DPD, 32,768 in 2,197 cells: 100 / 117; Morse,
     // 252,000 in 24 boxes, 12 to 16 a cell, edge 1.0 to 1.08: 302 / 300. Force pass: Lennard-Jones, 10 a
-    // cell, edge 1.0: 205 / 176; 20, edge 1.25: 231 / 169.
+    // cell, edge 1.0: 205 / 176; 20, edge 1.25: 231 / 169. The line lies above 4/3, where three or more cells
+    // of the cutoff always fit, so that an ensemble's replicas take one kernel: with the smallest of four
+    // (629 to 2,866 particles, its edge 1.23) by columns the two launches took a step 94 us, 79 with one.
     bool any_dpd = false, costly = false;
     for (const Space &sp : spaces)
         for (size_t k = 0; k < sp.pot_idx.size(); ++k)
@@ -1260,7 +1262,7 @@ int mxg_engine::start(cudaStream_t st) {
     costly = !any_dpd || costly || rng_mode != 0;
     for (size_t r = 0; r < spaces.size(); ++r) {
         const Space &sp = spaces[r];
-        const bool few_candidates = rep_parts[r] >= (any_dpd ? 8LL : 11LL) * sp.ncells && sp.h[2] < 1.2 * cutoff;
+        const bool few_candidates = rep_parts[r] >= (any_dpd ? 8LL : 11LL) * sp.ncells && sp.h[2] < 1.34 * cutoff;
         by_column[r] = recorded && sp.columns_apply(cutoff) && !(costly && few_candidates);
         const bool flux_columns = has_fluxes && sp.columns_apply(cutoff);
         hflux_columns[r] = flux_columns;
