@@ -1251,6 +1251,10 @@ int mxg_engine::start(cudaStream_t st) {
     // cell, edge 1.0: 205 / 176; 20, edge 1.25: 231 / 169. The line lies above 4/3, where three or more cells
     // of the cutoff always fit, so that an ensemble's replicas take one kernel: with the smallest of four
     // (629 to 2,866 particles, its edge 1.23) by columns the two launches took a step 94 us, 79 with one.
+    // Engines with species fluxes stay on the cell kernel: the sums' order moves positions in the last bit,
+    // and there that is no rounding any more. A particle that changes cells keeps its rates for a step, and one
+    // pair more or less at a cutoff carries decay. 50,021 particles of 4 a cell, five entries, a step: 197 us
+    // with the forces by columns, 218 so (the fluxes themselves go by columns in both).
     bool any_dpd = false, costly = false;
     for (const Space &sp : spaces)
         for (size_t k = 0; k < sp.pot_idx.size(); ++k)
@@ -1263,7 +1267,7 @@ int mxg_engine::start(cudaStream_t st) {
     for (size_t r = 0; r < spaces.size(); ++r) {
         const Space &sp = spaces[r];
         const bool few_candidates = rep_parts[r] >= (any_dpd ? 8LL : 11LL) * sp.ncells && sp.h[2] < 1.34 * cutoff;
-        by_column[r] = recorded && sp.columns_apply(cutoff) && !(costly && few_candidates);
+        by_column[r] = recorded && !has_fluxes && sp.columns_apply(cutoff) && !(costly && few_candidates);
         const bool flux_columns = has_fluxes && sp.columns_apply(cutoff);
         hflux_columns[r] = flux_columns;
         flux_cells = flux_cells || !flux_columns;
