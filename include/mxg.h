@@ -470,8 +470,9 @@ int mxg_engine_time_force(mxg_engine *e, int reps, double *ms);
  * each launch starts with a cold L2; ms[r] receives launch r's milliseconds. The forces of the
  * state are recomputed in full afterwards; the state is not advanced. */
 int mxg_engine_time_force_launches(mxg_engine *e, int reps, void *flush, size_t flush_bytes, double *ms);
-/* Pair statistics for the last force evaluation: candidate and interacting pair counts as the
- * reference's task list defines them (counted on the device when enabled). */
+/* Pair statistics of the current positions: candidate and interacting pair counts as the
+ * reference's task list defines them (the latter counted on the device). Changes no state: forces,
+ * energies, species rates and bonds stay those of the last pass. */
 int mxg_engine_pair_counts(mxg_engine *e, long long *candidates, long long *interacting);
 
 /* ---- allocation-free entry point ---- */

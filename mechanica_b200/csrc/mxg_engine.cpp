@@ -3016,14 +3016,13 @@ int mxg_engine_pair_counts(mxg_engine *e, long long *candidates, long long *inte
     if (candidates) *candidates = cand;
     if (interacting) {
         // one statistics launch of the cell kernel counts the interacting pairs
-        // (each pair once, in the reference's orientation)
+        // (each pair once, in the reference's orientation); it writes nothing else
         unsigned long long *d_cnt = nullptr;
         CUDA_TRY(cudaMalloc(&d_cnt, sizeof(unsigned long long)));
         CUDA_TRY(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned long long), e->stream));
         EngineView v = e->all_cells_view();
         v.pair_stats = d_cnt;
         launch_force(v, e->has_dpd, e->num_sms * 16, 1, false, e->stream);
-        e->enqueue_force(e->cur);  // and the complete forces of the state, as engine_force leaves them
         unsigned long long n = 0;
         CUDA_TRY(cudaMemcpyAsync(&n, d_cnt, sizeof(n), cudaMemcpyDeviceToHost, e->stream));
         CUDA_TRY(cudaStreamSynchronize(e->stream));
