@@ -278,7 +278,8 @@ struct EngineView {      // everything a kernel needs, passed by value
     int *ovf_list;           // movers beyond their destination's bucket this step: old slot (capacity nparts)
     int *ovf_count;          // entries of ovf_list (re-armed by the re-binning launch)
     // the column force kernel (spaces it applies to; the others' cells are in items)
-    const int4 *col_items;   // (first cell of a column, first group of 32 particles, group step, cells along z)
+    const int4 *col_items;   // (first cell of a part of a column, first group of 32 particles, group step,
+                             // that cell's place along z << 4 | cells of the part)
     int ncol_items;
     int *chunk_delta;        // per chunk of 1 << kChunkShift cells: movers in minus movers out this step
 };

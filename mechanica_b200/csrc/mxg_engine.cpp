@@ -1230,8 +1230,8 @@ int mxg_engine::start(cudaStream_t st) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         num_sms = sms;
     }
-    // The spaces the column force kernel covers have no items here: their columns are its items, a
-    // column's groups of 32 particles shared out over about as many warps as it has groups on
+    // The spaces the column force kernel covers have no items here: their columns, in parts of
+    // up to kColumnSpan cells, are its items, a part's groups of 32 particles shared out over about as many warps as it has groups on
     // average, and a few to spare (a warp that finds no group ends at once, one that finds several
     // takes them in turn).
     std::vector<char> by_column(spaces.size());
@@ -1272,14 +1272,17 @@ int mxg_engine::start(cudaStream_t st) {
         hflux_columns[r] = flux_columns;
         flux_cells = flux_cells || !flux_columns;
         if (!by_column[r] && !flux_columns) continue;
-        const int ncol = sp.cdim[0] * sp.cdim[1], cz = sp.cdim[2];
-        const double mean = (double)rep_parts[r] / ncol / 32.0;
+        const int ncol = sp.cdim[0] * sp.cdim[1], cz = sp.cdim[2], parts = (cz + kColumnSpan - 1) / kColumnSpan;
+        const double mean = (double)rep_parts[r] / ncol / parts / 32.0;
         const int step = std::max(1, (int)std::ceil(1.15 * mean + 0.5));
         for (int c = 0; c < ncol; ++c)
-            for (int g = 0; g < step; ++g) {
-                const int4 item = make_int4(sp.cell_offset + c * cz, g, step, cz);
-                if (by_column[r]) hcol.push_back(item);
-                if (flux_columns) hfluxcol.push_back(item);
+            for (int p = 0; p < parts; ++p) {
+                const int z = (int)((long long)cz * p / parts), cells = (int)((long long)cz * (p + 1) / parts) - z;
+                for (int g = 0; g < step; ++g) {
+                    const int4 item = make_int4(sp.cell_offset + c * cz + z, g, step, z << 4 | cells);
+                    if (by_column[r]) hcol.push_back(item);
+                    if (flux_columns) hfluxcol.push_back(item);
+                }
             }
     }
     ncol_items = (int)hcol.size();

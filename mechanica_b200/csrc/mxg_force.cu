@@ -22,7 +22,9 @@
  * Positions are staged as integers, units of a power of two near 2^-27 of a cell edge from the
  * middle of the warp's cells: cell-relative FP32 positions convert exactly down to that unit, the
  * shift of a neighbour cell is an addition without rounding, and a pair's displacement is the same
- * from both sides, up to its sign, to the bit. The arithmetic below is in these units.
+ * from both sides, up to its sign, to the bit. The arithmetic below is in these units. 32 bits hold
+ * the kColumnSpan cells that a warp's particles may span and those on both sides of them: longer
+ * columns are cut into parts of that length, so the unit is the same for every warp of a space.
  *
  * The sums' order is fixed by the column's own content, so results depend neither on scheduling nor
  * on what else is in the engine.
@@ -297,7 +299,7 @@ __device__ __forceinline__ void candidates(ColSmem<kKind> &sm, int u0, int base,
     for (int k = 0; k < 2 * kU; ++k) sm.mask[u0 + k][lane] = m[k];
 }
 
-/* z in the warp's frame; the sum may pass 2^31 on the way (at most 16 edges below 2^27 each). */
+/* z in the warp's frame; the sum may pass 2^31 on the way (at most kColumnSpan + 1 edges below 2^27 each). */
 __device__ __forceinline__ int column_z(int z, int cells, int edge, int off) {
     return (int)((unsigned)z + (unsigned)cells * (unsigned)edge + (unsigned)off);
 }
@@ -442,8 +444,8 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
     const int ntypes = v.ntypes;
     for (int it = blockIdx.x; it < v.ncol_items; it += gridDim.x) {
         const int4 item = v.col_items[it];
-        const int cell0 = item.x, cz = item.w;
-        const int slot0 = v.cell_start[cell0], n = v.cell_start[cell0 + cz] - slot0;
+        const int cell0 = item.x - (item.w >> 4);  // the column's first; the item's are at most kColumnSpan
+        const int slot0 = v.cell_start[item.x], n = v.cell_start[item.x + (item.w & 15)] - slot0;
         const int groups = (n + 31) >> 5;
         double energy = 0.0;
         for (int g = item.y; g < groups; g += item.z) {
@@ -461,10 +463,8 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             const int zlo = __shfl_sync(kFull, zi, 0), zhi = __shfl_sync(kFull, zi, nown - 1);
             int loc[3];
             cell_loc(S, cell0, loc);
-            // units: 2^26 to 2^27 a cell edge, half of it for each doubling of the cells along z past 15
-            const int shrink = max(0, 28 - __clz(zhi - zlo + 1));
-            const float unit = __int_as_float(__float_as_int(S.col_unit) + (shrink << 23));
-            const float scale = __int_as_float(__float_as_int(S.col_scale) - (shrink << 23));
+            const int cz = S.cdim[2];
+            const float unit = S.col_unit, scale = S.col_scale;  // 2^26 to 2^27 units a cell edge
             const int edge = __float2int_rn(S.h[2] * scale);  // a cell edge (the cells are cubic)
             const int zmid = (zhi - zlo + 1) * (edge >> 1) + edge;  // of the staged cells, one below zlo on
             own.zrel = zi - zlo;

@@ -28,6 +28,8 @@ void launch_bonded_virial(const EngineView &v, const BondedView &bv, int nb, int
 /* Forces of the spaces whose cells are cubic and no smaller than the cutoff (mxg_force.cu); split: 1, 4
  * or 8 warps per group of 32 particles; grid: blocks at most (an item each) */
 constexpr int kColumnParts = 8;     // energy rows per column item: the widest split's warps
+constexpr int kColumnSpan = 15;     // cells along z of an item at most (four bits): with the cells on both sides,
+                                    // coordinates in units of 2^-27 of an edge stay below 2^31
 void configure_column_kernels();
 void launch_column_force(const EngineView &v, bool has_dpd, int split, int grid, cudaStream_t st);
 /* Species fluxes of the spaces with DevSpace::flux_columns; v.col_items: their columns */
