@@ -1255,19 +1255,21 @@ int mxg_engine::start(cudaStream_t st) {
     // and there that is no rounding any more. A particle that changes cells keeps its rates for a step, and one
     // pair more or less at a cutoff carries decay. 50,021 particles of 4 a cell, five entries, a step: 197 us
     // with the forces by columns, 218 so (the fluxes themselves go by columns in both).
-    bool any_dpd = false, costly = false;
+    // In a DPD-only pass the columns take a force at the cutoff for zero, so one that reaches further stays here.
+    bool any_dpd = false, costly = false, fades = true;
     for (const Space &sp : spaces)
         for (size_t k = 0; k < sp.pot_idx.size(); ++k)
             for (int q : {sp.pot_idx[k], sp.pot2_idx[k]}) {
                 if (q < 0) continue;
                 any_dpd = any_dpd || pots[q].kind == kKindDPD;
+                fades = fades && !(pots[q].kind == kKindDPD && pots[q].b > cutoff * (1 + 1e-6));
                 costly = costly || pots[q].kind != kKindDPD || (pots[q].flags & kFlagShifted) || q == sp.pot2_idx[k];
             }
     costly = !any_dpd || costly || rng_mode != 0;
     for (size_t r = 0; r < spaces.size(); ++r) {
         const Space &sp = spaces[r];
         const bool few_candidates = rep_parts[r] >= (any_dpd ? 8LL : 11LL) * sp.ncells && sp.h[2] < 1.34 * cutoff;
-        by_column[r] = recorded && !has_fluxes && sp.columns_apply(cutoff) && !(costly && few_candidates);
+        by_column[r] = recorded && !has_fluxes && (fades || costly) && sp.columns_apply(cutoff) && !(costly && few_candidates);
         const bool flux_columns = has_fluxes && sp.columns_apply(cutoff);
         hflux_columns[r] = flux_columns;
         flux_cells = flux_cells || !flux_columns;
