@@ -266,12 +266,19 @@ struct EngineView {      // everything a kernel needs, passed by value
                              // random term, 2: the Philox stream
     int force_variant;       // the force kernel's tile shape (see Tile), chosen by the autotuner
     int nitems;
+    float near_r2;           // these three: see pair_rec
     const DevCuboid *cuboids;  // static cuboids (all replicas)
     int ncuboids;
+    float near_dpd;
     // per replica and type pair, the column kernel's record of the pair's potential and, if any is summed, of
-    // its second one: (a^2, m, c, b), (alpha0, alpha1, alpha2, interval count << 20 | first coefficient / 8)
-    // of a table at s = m r + c; (a^2, cutoff, 1 / cutoff, radii sum if shifted), (alpha, gamma, sigma delta,
-    // -1) of a DPD potential; a last word of -2: none
+    // its second one: (from, m, c, to), (alpha0, alpha1, alpha2, interval count << 20 | first coefficient / 8),
+    // (a^2, b, r0 + 1 if shifted, radii sum if shifted, less than zero if scaled) of a table at s = m r + c;
+    // (from, cutoff, 1 / cutoff, radii sum if shifted), (alpha, gamma, sigma delta, -1), (a^2, 0, 0, 0) of a
+    // DPD potential; a second part's last word of -2: none. from: the r^2 from which on no rounding decides whether
+    // the pair is closer than the potential's a (a^2 and near_r2 more), kClose2 of the cutoff squared at least;
+    // to: the r^2 up to which none decides whether it is past the table's end or the cutoff, and from to
+    // near_ratio times that one does (-1: no distance is in the table's range). near_dpd: from of the DPD
+    // potential with the largest a
     const float4 *pair_rec, *pair_rec2;
     const float4 *dpd_pair;  // DPD-only kernel, per replica and type pair: (rc, alpha, gamma, sigma delta),
                              // (a^2, a, 1/rc, alpha + sigma delta); null otherwise
@@ -281,6 +288,7 @@ struct EngineView {      // everything a kernel needs, passed by value
     const int4 *col_items;   // (first cell of a part of a column, first group of 32 particles, group step,
                              // that cell's place along z << 4 | cells of the part)
     int ncol_items;
+    float near_ratio;
     int *chunk_delta;        // per chunk of 1 << kChunkShift cells: movers in minus movers out this step
 };
 

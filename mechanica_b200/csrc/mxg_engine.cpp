@@ -538,8 +538,9 @@ struct mxg_engine {
     float *d_coef = nullptr;
     int *d_pot_idx = nullptr;
     int *d_pot_idx2 = nullptr;   // second summed potential per type pair, or -1
-    float4 *d_pair_rec = nullptr, *d_pair_rec2 = nullptr;  // column kernel: two records per replica and type pair
+    float4 *d_pair_rec = nullptr, *d_pair_rec2 = nullptr;  // column kernel: a record per replica and type pair
     float4 *d_dpd_pair = nullptr;  // DPD-only kernel: two records per replica and type pair
+    float near_ratio = 1.f;        // EngineView::near_ratio
     std::vector<int> h_pot_idx, h_pot_idx2;  // the device's potential indices per replica and type pair
     bool has_second = false;
     DevType *d_types = nullptr;
@@ -654,36 +655,83 @@ struct mxg_engine {
 
     /* The column kernel's records of the type pairs' potentials pidx (see EngineView::pair_rec). */
     std::vector<float4> pair_records(const std::vector<DevPot> &hp, const std::vector<int> &pidx) const {
-        std::vector<float4> out(std::max<size_t>(1, 2 * pidx.size()));
+        std::vector<float4> out(std::max<size_t>(1, 3 * pidx.size()));
         auto as_float = [](int x) {
             float f;
             memcpy(&f, &x, 4);
             return f;
         };
         const int tt = ntypes * ntypes;
+        const float close2 = kClose2 * (float)cutoff * (float)cutoff;
         for (size_t k = 0; k < pidx.size(); ++k) {
-            out[2 * k] = make_float4(0.f, 0.f, 0.f, -1e30f);  // no distance is in range
-            out[2 * k + 1] = make_float4(0.f, 0.f, 0.f, as_float(-2));
+            float4 *rec = &out[3 * k];
+            rec[0] = make_float4(0.f, 0.f, 0.f, -1.f);  // no distance is in range
+            rec[1] = make_float4(0.f, 0.f, 0.f, as_float(-2));
+            rec[2] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (pidx[k] < 0) continue;
             const DevPot &d = hp[pidx[k]];
             const int a = (int)(k % tt) / ntypes, b = (int)(k % tt) % ntypes;
-            const float rsum = (float)types[a].radius + (float)types[b].radius;
+            const float rsum = (float)types[a].radius + (float)types[b].radius, from = std::max(d.a2 + near_r2(), close2);
             if (d.kind == kKindDPD) {
                 const bool shifted = d.flags & kFlagShifted;
                 const float cut = shifted ? d.b + rsum : d.b;
-                out[2 * k] = make_float4(d.a2, cut, 1.0f / cut, shifted ? rsum : 0.f);
-                out[2 * k + 1] = make_float4(d.dpd_alpha, d.dpd_gamma, d.dpd_sigma * d.dpd_delta, as_float(-1));
+                rec[0] = make_float4(from, cut, 1.0f / cut, shifted ? rsum : 0.f);
+                rec[1] = make_float4(d.dpd_alpha, d.dpd_gamma, d.dpd_sigma * d.dpd_delta, as_float(-1));
+                rec[2].x = d.a2;
             } else {
                 const bool scaled = d.flags & kFlagScaled, shifted = !scaled && (d.flags & kFlagShifted);
-                out[2 * k] = make_float4(d.a2, scaled ? 1.0f / rsum : 1.0f, shifted ? d.r0_plusone - rsum : 0.f, d.b);
-                out[2 * k + 1] = make_float4(d.alpha0, d.alpha1, d.alpha2, as_float((int)((unsigned)d.n << 20 | (unsigned)(d.coef_off / kChunk))));
+                double lo, hi;
+                table_reach(pots[pidx[k]], rsum, lo, hi);
+                rec[0] = make_float4(from, scaled ? 1.0f / rsum : 1.0f, shifted ? d.r0_plusone - rsum : 0.f,
+                                     lo < 0 ? -1.f : (float)(lo * lo));
+                rec[1] = make_float4(d.alpha0, d.alpha1, d.alpha2, as_float((int)((unsigned)d.n << 20 | (unsigned)(d.coef_off / kChunk))));
+                rec[2] = make_float4(d.a2, d.b, shifted ? d.r0_plusone : 0.f, shifted ? rsum : scaled ? -rsum : 0.f);
             }
         }
         return out;
     }
+    float near_dpd() const {
+        float a2 = 0.f;
+        for (const auto &t : pots)
+            if (t.kind == kKindDPD) a2 = std::max(a2, t.a * t.a);
+        return std::max(a2 + near_r2(), kClose2 * (float)cutoff * (float)cutoff);
+    }
+    float near_r2() const { return near_cut() * (float)cutoff * (float)cutoff; }
 
-    /* Whether the records can hold every table (interval counts and places in the coefficient pool). */
-    bool records_hold() const {
+    /* The distances r between which rounding decides whether a pair is past the end of table t for types a and b
+     * (radii sum rsum) or past the cutoff, whichever is nearer: the displacements' width, and a few units in
+     * the last place of what the table's variable s = m r + c is formed from. lo < 0: none is in range. */
+    void table_reach(const mxg::PotentialTable &t, float rsum, double &lo, double &hi) const {
+        const bool scaled = t.flags & kFlagScaled, shifted = !scaled && (t.flags & kFlagShifted);
+        const double m = scaled ? 1.0 / rsum : 1.0, c = shifted ? (double)t.r0_plusone - rsum : 0.0, b = t.b;
+        const double wide = 0.5 * near_cut() * cutoff;
+        lo = cutoff - wide;
+        hi = cutoff + wide;
+        if (!std::isfinite(m)) {
+            lo = hi = -1.0;
+            return;
+        }
+        const double end = (b - c) / m, w = wide + 2.4e-7 * (cutoff + (std::fabs(b) + std::fabs(c)) / m);
+        lo = std::min(lo, end - w);
+        hi = std::min(hi, end + w);
+        if (hi >= 0 && lo < 0) lo = 0.0;
+    }
+
+    /* Whether the records can hold every table (interval counts, places in the coefficient pool, and ends that
+     * are not so near to zero that the width around them is no small part of it); ratio: EngineView::near_ratio. */
+    bool records_hold(float &ratio) const {
+        double widest = 1.0;
+        for (const Space &sp : spaces)
+            for (const std::vector<int> *idx : {&sp.pot_idx, &sp.pot2_idx})
+                for (int k = 0; k < (int)idx->size(); ++k) {
+                    const int q = (*idx)[k], a = k / max_type, b = k % max_type;
+                    if (q < 0 || pots[q].kind == kKindDPD) continue;
+                    double lo, hi;
+                    table_reach(pots[q], (float)types[a].radius + (float)types[b].radius, lo, hi);
+                    if (lo >= 0 && lo < cutoff / 64) return false;
+                    if (lo >= 0) widest = std::max(widest, hi / lo);
+                }
+        ratio = (float)(widest * widest * (1 + 2.4e-7));
         size_t intervals = 0;
         for (const auto &t : pots) {
             if (t.n >= 1 << 11) return false;
@@ -727,6 +775,13 @@ struct mxg_engine {
         int rc = dev_alloc(p, n);
         if (rc == MXG_OK) allocations.push_back((void *)*p);
         return rc;
+    }
+
+    float near_cut(const Space &sp) const { return (float)(4.0 * 2.4e-7 * 2.0 * std::max(cutoff, sp.h[2]) / cutoff); }
+    float near_cut() const {
+        float widest = 0.f;
+        for (const Space &sp : spaces) widest = std::max(widest, near_cut(sp));
+        return widest;
     }
 
     DevSpace space_desc(int r, int pot_offset) const {
@@ -780,7 +835,7 @@ struct mxg_engine {
         S.col_unit = std::ldexp(1.0f, exponent - 27);
         // displacements round at two cell edges in the reference, here at 2^-24 of themselves: twice that,
         // relative to the cutoff, for r^2, with a factor of two to spare
-        S.near_cut = (float)(4.0 * 2.4e-7 * 2.0 * std::max(cutoff, sp.h[2]) / cutoff);
+        S.near_cut = near_cut(sp);
         S.off_cell = integrator == 1 ? 1 : 0;
         S.sort_bias = sp.sort_bias();
         S.sort_dscale = sp.sort_dscale();
@@ -888,6 +943,9 @@ struct mxg_engine {
         v.dpd_pair = dpd_pure ? d_dpd_pair : nullptr;
         v.pair_rec = d_pair_rec;
         v.pair_rec2 = d_pair_rec2;
+        v.near_r2 = near_r2();
+        v.near_ratio = near_ratio;
+        v.near_dpd = near_dpd();
         v.chunk_delta = d_chunk_delta[b];
         v.ovf_list = d_ovf_list;
         v.ovf_count = d_ovf_count;
@@ -1240,7 +1298,7 @@ int mxg_engine::start(cudaStream_t st) {
     std::vector<int4> hcol, hfluxcol;
     std::vector<char> hflux_columns(spaces.size(), 0);
     flux_cells = false;
-    const bool recorded = records_hold();
+    const bool recorded = records_hold(near_ratio);
     // The cell kernel evaluates each pair once where the columns do it from both sides, so it keeps the
     // engines with costly pair terms while its candidates are few: cells of up to 1.34 cutoffs with 11
     // particles or more, 8 where a DPD term draws from the Philox stream or is summed with a table (below

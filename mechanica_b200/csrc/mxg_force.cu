@@ -74,8 +74,8 @@ struct PairRec {
 };
 __device__ __forceinline__ PairRec load_rec(const float4 *rec, int pk) {
     PairRec r;
-    r.p = __ldg(rec + 2 * pk);
-    r.q = __ldg(rec + 2 * pk + 1);
+    r.p = __ldg(rec + 3 * pk);
+    r.q = __ldg(rec + 3 * pk + 1);
     return r;
 }
 
@@ -86,9 +86,9 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return y;
 }
 
-/* Potential and force of a table at r2 >= a^2 (potential_eval_ex, potential_eval.hpp:106-161; e and
- * f = V'(r) / r): false out of range. Fused multiply-adds, and the square root and the division by r
- * from one reciprocal square root with a Newton step for r. */
+/* Potential and force of a table at r2 >= a^2 and not past its end (potential_eval_ex, potential_eval.hpp:
+ * 106-161; e and f = V'(r) / r): false out of range. Fused multiply-adds, and the square root and the
+ * division by r from one reciprocal square root with a Newton step for r. */
 __device__ __forceinline__ bool table_term(const PairRec &rec, const float *__restrict__ coef, float r2, float &e, float &f) {
     const float r2c = fmaxf(r2, 1.42108547e-14f);  // the reference's lower bound on r, FLT_EPSILON
     const float ir = rsqrt_ftz(r2c);
@@ -97,8 +97,8 @@ __device__ __forceinline__ bool table_term(const PairRec &rec, const float *__re
     const float s = __fmaf_rn(r, rec.p.y, rec.p.z);
     const float t = __fmaf_rn(s, __fmaf_rn(s, rec.q.z, rec.q.y), rec.q.x);
     const unsigned ind = (unsigned)fmaxf(0.0f, t);
-    const unsigned code = (unsigned)max(rec.code(), 0), count = code >> 20;  // without a potential b is -1e30
-    const bool in = s <= rec.p.w && ind <= count;  // no branch: the last interval's values are not used
+    const unsigned code = (unsigned)max(rec.code(), 0), count = code >> 20;
+    const bool in = ind <= count;  // no branch: the last interval's values are not used
     const float4 *c4 = reinterpret_cast<const float4 *>(coef) + 2 * ((code & 0xfffffu) + min(ind, count));
     const float4 c0 = __ldg(c4), c1 = __ldg(c4 + 1);
     const float x = __fmul_rn(__fsub_rn(s, c0.x), c0.y);
@@ -118,33 +118,73 @@ __device__ __forceinline__ float dpd_term(float oc, float ir, float dv, float ga
     return __fmul_rn(__fmul_rn(oc, __fmaf_rn(__fmul_rn(-gamma, oc), __fmul_rn(dv, ir), drive)), ir);
 }
 
-/* One term of a pair (rec its potential, d from the neighbour to the own particle): the own
+/* The DPD term of a pair (rec its potential, d from the neighbour to the own particle): the own
  * particle's force is fs * d. False out of range. */
-template <int kKind>
-__device__ __forceinline__ bool pair_term(const EngineView &v, const PairRec &rec, float dx, float dy, float dz, float r2,
-                                          const float4 &vi, const float4 &vj, unsigned rng_mode, float &fs, float &e) {
-    e = 0.f;
-    if (kKind != kTerms && rec.code() < 0) {
-        if (r2 > __fmul_rn(rec.p.y, rec.p.y) || rec.code() == -2) return false;
-        // r, 1/r and the quotient by the cutoff one Newton step on from the unit's results: as close to
-        // the FP64 values as divisions (DPD mixed with tables, shifted, or with the Philox stream)
-        float ir = rsqrt_ftz(r2);
-        float r = __fmul_rn(r2, ir);
-        r = __fmaf_rn(__fmaf_rn(-r, r, r2), 0.5f * ir, r);
-        ir = __fmaf_rn(__fmaf_rn(-r, ir, 1.0f), ir, ir);
-        const float sr = __fsub_rn(r, rec.p.w), qt = __fmul_rn(sr, rec.p.z);
-        const float oc = sr < 0.f ? 1.f : __fmaf_rn(__fmaf_rn(qt, rec.p.y, -sr), rec.p.z, __fsub_rn(1.0f, qt));
-        const float dv = __fmaf_rn(dx, __fsub_rn(vi.x, vj.x),
-                                   __fmaf_rn(dy, __fsub_rn(vi.y, vj.y), __fmul_rn(dz, __fsub_rn(vi.z, vj.z))));
-        float xi = 1.f;
-        if (rng_mode) {
-            const unsigned idi = __float_as_uint(vi.w), idj = __float_as_uint(vj.w);
-            xi = philox_pair_xi(*v.step, min(idi, idj), max(idi, idj));
-        }
-        fs = dpd_term(oc, ir, dv, rec.q.y, __fmaf_rn(rec.q.z, xi, rec.q.x));
-        return true;
+__device__ __forceinline__ bool pair_dpd(const EngineView &v, const PairRec &rec, float dx, float dy, float dz, float r2,
+                                         const float4 &vi, const float4 &vj, unsigned rng_mode, float &fs) {
+    if (r2 > __fmul_rn(rec.p.y, rec.p.y) || rec.code() == -2) return false;
+    // r, 1/r and the quotient by the cutoff one Newton step on from the unit's results: as close to
+    // the FP64 values as divisions (DPD mixed with tables, shifted, or with the Philox stream)
+    float ir = rsqrt_ftz(r2);
+    float r = __fmul_rn(r2, ir);
+    r = __fmaf_rn(__fmaf_rn(-r, r, r2), 0.5f * ir, r);
+    ir = __fmaf_rn(__fmaf_rn(-r, ir, 1.0f), ir, ir);
+    const float sr = __fsub_rn(r, rec.p.w), qt = __fmul_rn(sr, rec.p.z);
+    const float oc = sr < 0.f ? 1.f : __fmaf_rn(__fmaf_rn(qt, rec.p.y, -sr), rec.p.z, __fsub_rn(1.0f, qt));
+    const float dv = __fmaf_rn(dx, __fsub_rn(vi.x, vj.x),
+                               __fmaf_rn(dy, __fsub_rn(vi.y, vj.y), __fmul_rn(dz, __fsub_rn(vi.z, vj.z))));
+    float xi = 1.f;
+    if (rng_mode) {
+        const unsigned idi = __float_as_uint(vi.w), idj = __float_as_uint(vj.w);
+        xi = philox_pair_xi(*v.step, min(idi, idj), max(idi, idj));
     }
-    if (!table_term(rec, v.coef, r2, e, fs)) return false;
+    fs = dpd_term(oc, ir, dv, rec.q.y, __fmaf_rn(rec.q.z, xi, rec.q.x));
+    return true;
+}
+
+/* One term of a pair in an engine of tables and DPD: the own particle's force is fs * d. False out of
+ * range; edge: so near to a table's end that rounding decides on which side of it the pair is. */
+__device__ __forceinline__ bool pair_term(const EngineView &v, const PairRec &rec, float dx, float dy, float dz, float r2,
+                                          const float4 &vi, const float4 &vj, unsigned rng_mode, float &fs, float &e,
+                                          bool &edge) {
+    e = 0.f;
+    edge = false;
+    if (rec.code() < 0) return pair_dpd(v, rec, dx, dy, dz, r2, vi, vj, rng_mode, fs);
+    const bool in = table_term(rec, v.coef, r2, e, fs);
+    fs = -fs;
+    edge = r2 > rec.p.w && r2 <= rec.p.w * v.near_ratio;
+    return in && r2 <= rec.p.w;
+}
+
+/* potential_eval_ex in its own arithmetic, for the pairs of odd_pairs; x: the record's third part. It is
+ * loaded with the others: the chain of loads of one such pair is as long as the kernel's last warp. */
+__device__ __forceinline__ bool table_reference(const PairRec &rec, const float4 &x, const float *__restrict__ coef, float r2,
+                                                float &e, float &f) {
+    const float r = __fsqrt_rn(r2), ro = fmaxf(r, 1.19209290e-7f), ra = fmaxf(r, __fsqrt_rn(x.x));
+    const float s = x.w < 0.f ? __fdiv_rn(ra, -x.w) : __fadd_rn(__fsub_rn(ra, x.w), x.z);
+    const float t = __fadd_rn(rec.q.x, __fmul_rn(s, __fadd_rn(rec.q.y, __fmul_rn(s, rec.q.z))));
+    const unsigned ind = (unsigned)fmaxf(0.0f, t), code = (unsigned)rec.code();
+    if (s > x.y || ind > code >> 20) return false;
+    const float4 *c4 = reinterpret_cast<const float4 *>(coef) + 2 * ((code & 0xfffffu) + ind);
+    const float4 c0 = __ldg(c4), c1 = __ldg(c4 + 1);
+    const float u = __fmul_rn(__fsub_rn(s, c0.x), c0.y);
+    float ee = __fadd_rn(__fmul_rn(c0.z, u), c0.w), eff = c0.z;
+    eff = __fadd_rn(__fmul_rn(eff, u), ee); ee = __fadd_rn(__fmul_rn(ee, u), c1.x);
+    eff = __fadd_rn(__fmul_rn(eff, u), ee); ee = __fadd_rn(__fmul_rn(ee, u), c1.y);
+    eff = __fadd_rn(__fmul_rn(eff, u), ee); ee = __fadd_rn(__fmul_rn(ee, u), c1.z);
+    eff = __fadd_rn(__fmul_rn(eff, u), ee); ee = __fadd_rn(__fmul_rn(ee, u), c1.w);
+    e = ee;
+    f = __fdiv_rn(__fmul_rn(eff, c0.y), ro);
+    return true;
+}
+
+/* pair_term for the pairs of odd_pairs. */
+template <int kKind>
+__device__ __forceinline__ bool odd_term(const EngineView &v, const PairRec &rec, const float4 &x, const float3 &d, float r2,
+                                         const float4 &vi, const float4 &vj, unsigned rng_mode, float &fs, float &e) {
+    e = 0.f;
+    if (kKind != kTerms && rec.code() < 0) return pair_dpd(v, rec, d.x, d.y, d.z, r2, vi, vj, rng_mode, fs);
+    if (kKind == kTermsPureDpd || !table_reference(rec, x, v.coef, r2, e, fs)) return false;
     fs = -fs;
     return true;
 }
@@ -339,16 +379,11 @@ __device__ __noinline__ bool reference_within(const EngineView &v, const DevSpac
     return dot3_rn(d.x, d.y, d.z) <= (side == 0 ? S.cut2_self : S.cut2_pair);
 }
 
-/* Closer than 1/64 of the cutoff (r^2 as a fraction of its square), the last bit of a position turns a
- * pair's direction by 4e-6 and more: such pairs, one particle in 5,000 at twelve in a cell, take the
- * reference's displacement too. */
-constexpr float kClose2 = 1.0f / 4096.0f;
-
 /* The pairs that the main walk leaves out: those closer than their potential's a, which get a random
- * direction of that length, those so near to a or to the cutoff that the decision depends on rounding
- * (in a DPD-only pass the force vanishes at the cutoff, and only a counts), and those closer than
- * kClose2. They take the reference's displacement, r^2 unfused. The main walk clears a lane's bits as it
- * takes them and sets these again; rare, so a walk of its own. */
+ * direction of that length, those so near to a, to the cutoff or to a table's end that the decision depends
+ * on rounding (in a DPD-only pass the force vanishes at the cutoff, and only a counts), and those closer
+ * than kClose2. They take the reference's displacement, r^2 unfused, and its evaluation of a table. The main
+ * walk clears a lane's bits as it takes them and sets these again; rare, so a walk of its own. */
 template <int kKind>
 __device__ __noinline__ ColSums odd_pairs(const EngineView &v, ColSmem<kKind> &sm, const DevSpace &S, ColOwn o, int x, int y,
                                           int z, int ngroups, bool live) {
@@ -363,6 +398,7 @@ __device__ __noinline__ ColSums odd_pairs(const EngineView &v, ColSmem<kKind> &s
             const int pk = S.pot_offset + o.type * v.ntypes + (b.w & 63);
             const PairRec rec = load_rec(v.pair_rec, pk);
             if (rec.code() == -2) continue;
+            const float4 x3 = __ldg(v.pair_rec + 3 * pk + 2);
             const int slot_j = kKind == kTermsPureDpd ? v.slot_of_id[__float_as_int(sm.nb_v[jj].w)] : sm.slot[jj];
             const int c9 = ((b.w >> 6) & 31) % 9, oz = (b.w >> 11) - 1 - o.zrel;
             const int side = (c9 / 3 - 1) * 9 + (c9 % 3 - 1) * 3 + oz;  // 0: own cell, > 0: the first of the two
@@ -372,21 +408,21 @@ __device__ __noinline__ ColSums odd_pairs(const EngineView &v, ColSmem<kKind> &s
             if (r2 > cut2) continue;
             const float4 vj = kKind != kTerms ? sm.nb_v[jj] : make_float4(0.f, 0.f, 0.f, 0.f);
             float3 t = d;
-            if (r2 < rec.p.x) {
+            if (r2 < x3.x) {
                 const unsigned idi = __float_as_uint(kKind != kTerms ? o.vel.w : v.vel[o.slot].w);
                 const unsigned idj = __float_as_uint(kKind != kTerms ? vj.w : v.vel[sm.slot[jj]].w);
-                t = close_pair(v, idi, idj, sqrtf(rec.p.x));
+                t = close_pair(v, idi, idj, sqrtf(x3.x));
             }
             float fs = 0.f, e = 0.f;
-            if (!pair_term<kKind>(v, rec, t.x, t.y, t.z, fmaxf(r2, rec.p.x), o.vel, vj, S.rng_mode, fs, e)) fs = e = 0.f;
+            if (!odd_term<kKind>(v, rec, x3, t, fmaxf(r2, x3.x), o.vel, vj, S.rng_mode, fs, e)) fs = e = 0.f;
             sum.x += fs * t.x;
             sum.y += fs * t.y;
             sum.z += fs * t.z;
             sum.e += (double)e;
             if (kKind == kTermsDpd && v.pot_idx2) {  // a second potential acts on the pair's own displacement
                 const PairRec rec2 = load_rec(v.pair_rec2, pk);
-                if (rec2.code() != -2 && !(r2 < rec2.p.x) &&
-                    pair_term<kKind>(v, rec2, d.x, d.y, d.z, r2, o.vel, vj, S.rng_mode, fs, e)) {
+                const float4 y3 = __ldg(v.pair_rec2 + 3 * pk + 2);
+                if (rec2.code() != -2 && !(r2 < y3.x) && odd_term<kKind>(v, rec2, y3, d, r2, o.vel, vj, S.rng_mode, fs, e)) {
                     sum.x += fs * d.x;
                     sum.y += fs * d.y;
                     sum.z += fs * d.z;
@@ -471,7 +507,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             own.x = __float2int_rn(xi.x * scale) - (edge >> 1);
             own.y = __float2int_rn(xi.y * scale) - (edge >> 1);
             own.z = column_z(__float2int_rn(xi.z * scale), zi - zlo + 1, edge, -zmid);
-            // pairs within a rounding of the cutoff, or of their potential's a, go to odd_pairs
+            // pairs within a rounding of the cutoff, of their potential's a or of a table's end go to odd_pairs
             const float cut2 = S.cut2_pair * scale * scale * (1.f + S.near_cut), cut2_in = S.cut2_pair * scale * scale * (1.f - S.near_cut);
             float blo[3], bhi[3], reach2;
             {
@@ -558,7 +594,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             constexpr int kBatch = needs_velocities(kKind) ? 3 : 2;  // rounds of 32 loaded together: more cost registers
             const int pair_base = S.pot_offset + own.type * ntypes;
             const unsigned rng_mode = S.rng_mode;
-            const float wide = 1.f + S.near_cut, close2 = kClose2 * S.cut2_pair;
+            const float near2 = v.near_dpd * (scale * scale);
             const double inv_cutoff = 1.0 / S.cutoff_d;
             float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
             if (kKind == kTermsPureDpd && one_type) {
@@ -716,38 +752,47 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                         const float oc = fmaxf(__fmaf_rn(-__fmul_rn(s2, ir), q1.z * unit, 1.0f), 0.f);
                         const float dv = __fmaf_rn(dx, own.vel.x - vj.x, __fmaf_rn(dy, own.vel.y - vj.y, dz * (own.vel.z - vj.z)));
                         fs = dpd_term(oc, ir, dv, q0.z, q1.w);
-                        const bool near = s2 < fmaxf(q1.x, close2) * (scale * scale);  // than a, or for the direction
+                        // than a, or for the direction
+                        const bool near = s2 < near2;
                         if (near && within) later(jj);
                         fs = within && !near ? fs : 0.f;
                     } else {
                         const int pk = pair_base + (b.w & 63);
                         if (!one_type) rec = load_rec(v.pair_rec, pk);
                         const float r2 = s2 * (unit * unit);
-                        const bool use = s2 <= cut2_in && r2 >= fmaxf(rec.p.x * wide, close2);
+                        // from past a to before the table's end or the cutoff
+                        bool use = r2 >= rec.p.x && (kKind == kTerms ? r2 <= rec.p.w : s2 <= cut2_in);
+                        const bool met = kKind == kTerms ? r2 <= rec.p.w * v.near_ratio : within;
                         float e;
-                        bool in;
                         tx = dx * unit;
                         ty = dy * unit;
                         tz = dz * unit;
                         if (kKind == kTerms) {
-                            in = table_term(rec, v.coef, r2, e, fs) && use;
+                            const bool in = table_term(rec, v.coef, r2, e, fs) && use;
                             fs = in ? -fs : 0.f;
                             e = in ? e : 0.f;
                         } else {
                             fs = e = 0.f;
-                            in = use && pair_term<kKind>(v, rec, tx, ty, tz, r2, own.vel, sm.nb_v[jj], rng_mode, fs, e);
-                            if (!in) fs = e = 0.f;
-                            if (v.pot_idx2 && use) {  // a second potential summed on the pair
-                                const PairRec rec2 = load_rec(v.pair_rec2, pk);
-                                float f2 = 0.f, e2 = 0.f;
-                                if (rec2.code() != -2 && !(r2 < rec2.p.x) &&
-                                    pair_term<kKind>(v, rec2, tx, ty, tz, r2, own.vel, sm.nb_v[jj], rng_mode, f2, e2)) {
-                                    fs += f2;
-                                    e += e2;
+                            if (use) {
+                                bool edge;
+                                if (!pair_term(v, rec, tx, ty, tz, r2, own.vel, sm.nb_v[jj], rng_mode, fs, e, edge))
+                                    fs = e = 0.f;
+                                use = !edge;
+                                if (v.pot_idx2) {  // a second potential summed on the pair
+                                    const PairRec rec2 = load_rec(v.pair_rec2, pk);
+                                    float f2 = 0.f, e2 = 0.f;
+                                    if (rec2.code() != -2 && !(r2 < rec2.p.x - 2.f * v.near_r2)) {
+                                        if (pair_term(v, rec2, tx, ty, tz, r2, own.vel, sm.nb_v[jj], rng_mode, f2, e2, edge)) {
+                                            fs += f2;
+                                            e += e2;
+                                        }
+                                        use = use && !edge && r2 >= rec2.p.x;
+                                    }
                                 }
+                                if (!use) fs = e = 0.f;
                             }
                         }
-                        if (within && !use) later(jj);
+                        if (met && !use) later(jj);
                         sum.e += (double)e;
                     }
                     sum.x = __fmaf_rn(fs, tx, sum.x);

@@ -30,6 +30,10 @@ void launch_bonded_virial(const EngineView &v, const BondedView &bv, int nb, int
 constexpr int kColumnParts = 8;     // energy rows per column item: the widest split's warps
 constexpr int kColumnSpan = 15;     // cells along z of an item at most (four bits): with the cells on both sides,
                                     // coordinates in units of 2^-27 of an edge stay below 2^31
+/* Closer than 1/64 of the cutoff (r^2 as a fraction of its square), the last bit of a position turns a
+ * pair's direction by 4e-6 and more: such pairs, one particle in 5,000 at twelve in a cell, take the
+ * reference's displacement there. */
+constexpr float kClose2 = 1.0f / 4096.0f;
 void configure_column_kernels();
 void launch_column_force(const EngineView &v, bool has_dpd, int split, int grid, cudaStream_t st);
 /* Species fluxes of the spaces with DevSpace::flux_columns; v.col_items: their columns */

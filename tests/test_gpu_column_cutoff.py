@@ -1,7 +1,8 @@
-"""Decisions of a force pass that hang on the last bits of the positions, by the reference's FP32 arithmetic (the
+"""Decisions of a column pass that hang on the last bits of the positions, by the reference's FP32 arithmetic (the
 oracle decides with it): isolated pairs within a few units in the last place of the cutoff where the force does
-not vanish, across faces of the cells and of the periodic box. Each force is the pair's in full or not there at
-all."""
+not vanish, of a table's own end inside the cutoff (shifted, scaled, summed with a DPD term), of a table's start
+and of a summed second table's start; across faces of the cells and of the periodic box. Each force is the pair's
+in full or not there at all."""
 import numpy as np
 import pytest
 
@@ -36,6 +37,13 @@ CASES = {
     "cutoff, with a DPD term": (_one(_morse, _dpd), 0.7, lambda p: 1.0),
     "cutoff, two types": (_mixed(_morse, lambda: _dpd(1.5)), 0.7, lambda p: 1.0),
     "cutoff, DPD that reaches further": (_one(lambda: _dpd(1.5)), 0.7, lambda p: 1.0),
+    "end of a shifted table": (_one(lambda: _morse(hi=1.15)), 0.7, lambda p: p.max - p._info()["r0_plusone"] + 1.4),
+    "end, with a DPD term": (_one(lambda: _morse(hi=1.15), _dpd), 0.7, lambda p: p.max - p._info()["r0_plusone"] + 1.4),
+    "end of a short shifted table": (_one(lambda: _morse(hi=0.6)), 0.7, lambda p: p.max - p._info()["r0_plusone"] + 1.4),
+    "end of a scaled table": (_one(lambda: m.Potential.power(10.0, 1.0, 2.0, 0.05, 1.8, 1e-3)), 0.25, lambda p: p.max * 0.5),
+    "start of a table": (_one(lambda: _morse(lo=0.1)), 0.7, lambda p: p.min),
+    "start, with a DPD term": (_one(lambda: _morse(lo=0.3), _dpd), 0.7, lambda p: p.min),
+    "start of a second table": (_one(_dpd, lambda: _morse(lo=0.3)), 0.7, None),
 }
 
 
@@ -44,7 +52,7 @@ CASES = {
 def test_decisions_follow_the_reference(name, variant):
     make, radius, where = CASES[name]
     pots, ntypes = make()
-    r0 = where(pots[0][0])
+    r0 = pots[0][1].min if where is None else where(pots[0][0])
     rng = np.random.default_rng(len(name))
     cell = np.stack(np.meshgrid(*[np.arange(0, SIDE, 3)] * 3, indexing="ij"), -1).reshape(-1, 3)
     n = len(cell)
@@ -91,7 +99,19 @@ def test_decisions_follow_the_reference(name, variant):
     assert np.array_equal(f[:n], -f[n:])
     big = np.abs(f64).max()
     on = np.abs(f64[:n]).max(axis=1)
+    if "start" in name and "second" not in name:
+        # a pair closer than the start gets a random direction, and none from the oracle's table; with a DPD term
+        # that one alone is there
+        d = (xr[:n].astype(np.float64) + np.stack([c[:n] // 144, c[:n] // 12 % 12, c[:n] % 12], -1)) - (
+            xr[n:].astype(np.float64) + np.stack([c[n:] // 144, c[n:] // 12 % 12, c[n:] % 12], -1))
+        d -= SIDE * np.round(d / SIDE)
+        h = np.linalg.norm(np.cross(f[:n], d), axis=1) / (np.linalg.norm(f[:n], axis=1) * np.linalg.norm(d, axis=1))
+        direct = on > 0.5 * big / np.sqrt(3)
+        assert 0 < direct.sum() < n
+        assert h[direct].max() <= 1e-5 < h[~direct].min()
+        assert np.abs(f[:n] - f64[:n])[direct].max() <= 1e-5 * big
+        return
     decided = on[on > 0]
-    if "DPD term" not in name and "two types" not in name:
+    if "DPD term" not in name and "two types" not in name and "second" not in name:
         assert 0 < len(decided) < n
     assert np.abs(f - f64).max() <= 1e-5 * big
