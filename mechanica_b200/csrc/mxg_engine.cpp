@@ -768,6 +768,7 @@ struct mxg_engine {
             coef.insert(coef.end(), t.c.begin(), t.c.end());
             hp.push_back(d);
         }
+        if (coef.empty()) coef.resize(kChunk, 0.f);  // pairs without a potential read the first interval
     }
 
     template <typename T>
