@@ -457,10 +457,11 @@ __device__ __forceinline__ void pair_fluxes(const EngineView &v, const SpeciesVi
         float g;
         if (F.kind == 0)
             g = __fmul_rn(F.k, __fsub_rn(sa, sb));
-        else if (F.kind == 1)
-            g = fmaxf(__fmul_rn(F.k, __fsub_rn(sa, F.target)), 0.f);
-        else
-            g = fmaxf(__fmul_rn(__fmul_rn(F.k, __fsub_rn(F.target, sb)), sa), 0.f);
+        else {  // times 0 or 1, so that values that are not finite reach both particles
+            const float u = F.kind == 1 ? __fmul_rn(F.k, __fsub_rn(sa, F.target))
+                                        : __fmul_rn(__fmul_rn(F.k, __fsub_rn(F.target, sb)), sa);
+            g = __fmul_rn(u > 0.f ? 1.f : 0.f, u);
+        }
         const float qq = __fmul_rn(w, g), hd = __fmul_rn(F.decay, 0.5f);
         if (ida == id) sm.rate[F.ia][lane] = __fsub_rn(__fsub_rn(sm.rate[F.ia][lane], qq), __fmul_rn(hd, sa));
         if (idb == id) sm.rate[F.ib][lane] = __fsub_rn(__fadd_rn(sm.rate[F.ib][lane], qq), __fmul_rn(hd, sb));

@@ -1,0 +1,36 @@
+"""Values that are not finite: a species value reaches the partner of a flux in both directions."""
+import numpy as np
+import pytest
+
+import mechanica_b200 as m
+from mechanica_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_fluxes_pass_on_what_is_not_finite(kind, value):
+    """Fick, secretion and uptake of one species between two types: the column kernel against the formula, 0 or 1
+    times the driving force, in numpy."""
+    x = np.array([[1.2, 1.5, 1.5], [1.7, 1.5, 1.5]])
+    k, target, dt = 2.0, 0.5, 0.01
+    for ill in (0, 1):
+        s = np.array([0.3, 0.4], dtype=np.float32)
+        s[ill] = value
+        u = W.build_gpu(dict(dim=[4.0] * 3, cells=[4] * 3, cutoff=1.0, dt=dt, bc=("periodic",) * 3,
+                             types=[(1.0, 0.1, m.Newtonian)] * 2, pots=[], forces=[], x=x, v=np.zeros((2, 3), np.float32),
+                             t=np.array([0, 1], dtype=np.int32), sp_nspec=np.array([1, 1], dtype=np.int32),
+                             sp_names=[["S1"], ["S1"]], sp_flags=np.zeros((2, 1), dtype=np.uint32),
+                             sp_values=s.reshape(2, 1), fluxes=[(kind, 0, 1, 0, 0, k, 0.0, target)]))
+        u.steps(1)
+        got = np.asarray(u.species_values()).ravel()
+        u.close()
+        with np.errstate(invalid="ignore"):
+            a, b = s.astype(np.float64)
+            drive = k * (a - b) if kind == 0 else k * (a - target) if kind == 1 else k * (target - b) * a
+            g = drive if kind == 0 else float(drive > 0) * drive
+            want = np.array([a - dt * (0.25 * g + 0.0 * a), b + dt * (0.25 * g - 0.0 * b)])  # no decay: 0 times the value
+        assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
+        fine = np.isfinite(want)
+        assert np.abs(got[fine] - want[fine]).max(initial=0.0) <= 1e-6
