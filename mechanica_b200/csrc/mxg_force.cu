@@ -344,6 +344,10 @@ __device__ __forceinline__ int column_z(int z, int cells, int edge, int off) {
     return (int)((unsigned)z + (unsigned)cells * (unsigned)edge + (unsigned)off);
 }
 
+/* Whether a cell-relative position is finite and near enough to its cell (7 edges, far) for its integer
+ * form, which has no other value for the rest; a particle that is not has no neighbours. */
+__device__ __forceinline__ bool on_grid(const float4 &x, float far) { return fabsf(x.x) + fabsf(x.y) + fabsf(x.z) <= far; }
+
 /* A lane's sums over the pairs it walks. */
 struct ColSums {
     float x, y, z;
@@ -503,6 +507,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
             const int cz = S.cdim[2];
             const float unit = S.col_unit, scale = S.col_scale;  // 2^26 to 2^27 units a cell edge
             const int edge = __float2int_rn(S.h[2] * scale);  // a cell edge (the cells are cubic)
+            const float far = 7.f * S.h[2];
             const int zmid = (zhi - zlo + 1) * (edge >> 1) + edge;  // of the staged cells, one below zlo on
             own.zrel = zi - zlo;
             own.x = __float2int_rn(xi.x * scale) - (edge >> 1);
@@ -518,9 +523,9 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                 reach2 = fmaxf(S.cut2w_pair, S.cut2w_self) * scale * scale + 2e-6f * (4.5f * ef * ef + ez * ez);
                 __syncwarp();
                 sm.own_xy[lane] = make_ulonglong2(pack2(-2.f * p[0], -2.f * p[0]), pack2(-2.f * p[1], -2.f * p[1]));
-                sm.own_zr[lane] =
-                    make_ulonglong2(pack2(-2.f * p[2], -2.f * p[2]),
-                                    pack2(reach2 - __fmaf_rn(p[0], p[0], __fmaf_rn(p[1], p[1], p[2] * p[2])), 0.f));
+                const float side = on_grid(xi, far) ? reach2 - __fmaf_rn(p[0], p[0], __fmaf_rn(p[1], p[1], p[2] * p[2]))
+                                                    : __int_as_float(0xff800000);
+                sm.own_zr[lane] = make_ulonglong2(pack2(-2.f * p[2], -2.f * p[2]), pack2(side, 0.f));
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     const int q = k == 0 ? own.x : k == 1 ? own.y : own.z;
@@ -659,7 +664,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                             const float ex = fmaxf(fmaxf(blo[0] - px, px - bhi[0]), 0.f);
                             const float ey = fmaxf(fmaxf(blo[1] - py, py - bhi[1]), 0.f);
                             const float ez = fmaxf(fmaxf(blo[2] - pz, pz - bhi[2]), 0.f);
-                            keep = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, ez * ez)) <= reach2;
+                            keep = __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, ez * ez)) <= reach2 && on_grid(q[r], far);
                         }
                         const unsigned bal = __ballot_sync(kFull, keep);
                         if (keep) {

@@ -1,4 +1,5 @@
-"""Values that are not finite: a species value reaches the partner of a flux in both directions."""
+"""Values that are not finite: a species value reaches the partner of a flux in both directions, and a particle
+whose position is lost no longer acts on its neighbours."""
 import numpy as np
 import pytest
 
@@ -34,3 +35,26 @@ def test_fluxes_pass_on_what_is_not_finite(kind, value):
         assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isinf(got), np.isinf(want))
         fine = np.isfinite(want)
         assert np.abs(got[fine] - want[fine]).max(initial=0.0) <= 1e-6
+
+
+POTENTIALS = [("dpd", (25.0, 4.5, 3.0, 1.0, 0)), ("morse", (0.5, 5.0, 1.0, 1e-4, 3.0, 1e-3))]
+
+
+@pytest.mark.parametrize("potential", POTENTIALS, ids=lambda p: p[0])
+@pytest.mark.parametrize("variant", [1, 3])
+def test_a_lost_particle_acts_on_nobody(potential, variant):
+    """One particle alone with a lost one beside it: after the step that loses it, it moves freely."""
+    x = np.array([[1.3, 1.4, 1.5], [1.6, 1.6, 1.6]])
+    u = W.build_gpu(dict(dim=[4.0] * 3, cells=[4] * 3, cutoff=1.0, dt=1e-4, bc=("periodic",) * 3,
+                         types=[(1.0, 0.1, m.Newtonian)] * 2, pots=[(*potential, 0, 1)],
+                         forces=[(1, float("nan"), 0.0, 0.0)], x=x, v=np.zeros((2, 3), np.float32),
+                         t=np.array([0, 1], dtype=np.int32)))
+    u.force_config(variant, 1 << 20)
+    with pytest.raises(m.EngineError):
+        u.steps(1)
+    v1 = u.velocities[0].copy()
+    assert np.isfinite(v1).all() and np.abs(v1).max() > 0 and not np.isfinite(u.positions[1]).all()
+    with pytest.raises(m.EngineError):
+        u.steps(5)
+    assert np.array_equal(u.velocities[0], v1)
+    u.close()
