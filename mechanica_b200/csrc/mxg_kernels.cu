@@ -2428,10 +2428,13 @@ __global__ void __launch_bounds__(kThreads, 1280 / kThreads) scatter_kernel(
             const DevSpace &S = v.spaces[s_rep[l]];
             if (!(S.prune & 2)) continue;
             const float bias = S.sort_bias, dscale = S.sort_dscale;
-            // the key does not fall as the projection rises: one conversion a bound
+            // the key does not fall as the projection rises: one conversion a bound. A projection that has no
+            // key counts as key 0, as in cell_sort_bounds
             float lo = INFINITY, hi = -INFINITY;
+            const float top = __fdiv_rn(2147483648.f, dscale);
             auto add = [&](const float4 &q) {
-                const float proj = sort_projection(q.x, q.y, q.z, n, bias);
+                float proj = sort_projection(q.x, q.y, q.z, n, bias);
+                proj = proj < top ? proj : -INFINITY;
                 lo = fminf(lo, proj);
                 hi = fmaxf(hi, proj);
             };

@@ -1,10 +1,12 @@
-"""Values that are not finite: a species value reaches the partner of a flux in both directions, and a particle
-whose position is lost no longer acts on its neighbours."""
+"""Values that are not finite: a species value reaches the partner of a flux in both directions, a particle whose
+position is lost no longer acts on its neighbours, and the key bounds of its cell are the same after a step as
+after a restore."""
 import numpy as np
 import pytest
 
 import mechanica_b200 as m
 from mechanica_b200 import workloads as W
+from mechanica_b200._native import check, lib
 
 pytestmark = pytest.mark.gpu
 
@@ -37,6 +39,16 @@ def test_fluxes_pass_on_what_is_not_finite(kind, value):
         assert np.abs(got[fine] - want[fine]).max(initial=0.0) <= 1e-6
 
 
+def _lost(n, rng, potential):
+    """A fluid in which the particles of type 1 lose their positions in the first step."""
+    x = rng.uniform(0, 4, size=(n, 3)).astype(np.float32).astype(np.float64)
+    t = np.zeros(n, dtype=np.int32)
+    t[::40] = 1
+    return W.build_gpu(dict(dim=[4.0] * 3, cells=[4] * 3, cutoff=1.0, dt=1e-4, bc=("periodic",) * 3,
+                            types=[(1.0, 0.1, m.Newtonian)] * 2, pots=[(*potential, 0, 0), (*potential, 0, 1)],
+                            forces=[(1, float("nan"), 0.0, 0.0)], x=x, v=np.zeros((n, 3), np.float32), t=t)), t
+
+
 POTENTIALS = [("dpd", (25.0, 4.5, 3.0, 1.0, 0)), ("morse", (0.5, 5.0, 1.0, 1e-4, 3.0, 1e-3))]
 
 
@@ -57,4 +69,24 @@ def test_a_lost_particle_acts_on_nobody(potential, variant):
     with pytest.raises(m.EngineError):
         u.steps(5)
     assert np.array_equal(u.velocities[0], v1)
+    u.close()
+
+
+@pytest.mark.parametrize("potential", POTENTIALS, ids=lambda p: p[0])
+def test_restore_after_a_loss(potential):
+    u, t = _lost(1200, np.random.default_rng(3), potential)
+    with pytest.raises(m.EngineError):
+        u.steps(2)
+    check(lib().mxg_engine_clear_status(u.handle), "clear_status")
+    ck = u.checkpoint()
+    with pytest.raises(m.EngineError):
+        u.steps(2)
+    a = [k.copy() for k in u.state()]
+    check(lib().mxg_engine_clear_status(u.handle), "clear_status")
+    u.restore(ck)
+    with pytest.raises(m.EngineError):
+        u.steps(2)
+    for p, q in zip(a, u.state()):
+        assert np.array_equal(p, q, equal_nan=True)
+    assert np.isfinite(a[1][t == 0]).all()
     u.close()
