@@ -710,6 +710,7 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                 int gbase = 0;
                 bool odd = false;
                 ColSums sum = {0.f, 0.f, 0.f, 0.0};  // of this region: shorter chains of FP32 additions
+                unsigned long long sx = 0ull, sy = 0ull, sz = 0ull;  // two sums each, of every other pair
                 // the next neighbour's staged index, or the place past the last, beyond any reach
                 auto next = [&]() -> int {
                     if (bits == 0u && some) {
@@ -727,12 +728,16 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                     sm.mask[jj >> 5][lane] |= 1u << (jj & 31);
                     odd = true;
                 };
-                auto pair = [&](int jj) {
+                // a pair's force is fs * (tx, ty, tz)
+                auto pair = [&](int jj, float &fs, float &tx, float &ty, float &tz) {
                     const int4 b = sm.nb[jj];
                     const float dx = (float)(own.x - b.x), dy = (float)(own.y - b.y), dz = (float)(own.z - b.z);
                     const float s2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));  // r^2 in units^2
                     const bool within = s2 <= cut2;
-                    float fs = 0.f, tx = dx, ty = dy, tz = dz;
+                    fs = 0.f;
+                    tx = dx;
+                    ty = dy;
+                    tz = dz;
                     if constexpr (kKind == kTermsFlux) {
                         if (!within) return;
                         const float r = fminf(__fsqrt_rn(s2) * unit, (float)S.cutoff_d);
@@ -801,17 +806,27 @@ __global__ void __launch_bounds__(32 * kSplit, 18 / kSplit) column_force_kernel(
                         if (met && !use) later(jj);
                         sum.e += (double)e;
                     }
-                    sum.x = __fmaf_rn(fs, tx, sum.x);
-                    sum.y = __fmaf_rn(fs, ty, sum.y);
-                    sum.z = __fmaf_rn(fs, tz, sum.z);
                 };
                 // two neighbours at a time without branches between them, so that their loads and arithmetic
                 // overlap
 #pragma unroll 1
                 for (int k = 0; k < most; k += 2) {
                     const int ja = next(), jb = next();
-                    pair(ja);
-                    pair(jb);
+                    float fa, xa, ya, za, fb, xb, yb, zb;
+                    pair(ja, fa, xa, ya, za);
+                    pair(jb, fb, xb, yb, zb);
+                    if (kKind != kTermsFlux) {
+                        const unsigned long long f2 = pack2(fa, fb);
+                        sx = fma2(f2, pack2(xa, xb), sx);
+                        sy = fma2(f2, pack2(ya, yb), sy);
+                        sz = fma2(f2, pack2(za, zb), sz);
+                    }
+                }
+                if (kKind != kTermsFlux) {
+                    const float2 px = unpack2(sx), py = unpack2(sy), pz = unpack2(sz);
+                    sum.x = px.x + px.y;
+                    sum.y = py.x + py.y;
+                    sum.z = pz.x + pz.y;
                 }
                 if (kKind != kTermsFlux && __any_sync(kFull, odd)) {
                     const ColSums c = odd_pairs<kKind>(v, sm, S, own, loc[0], loc[1], zi, ngrp, live);
