@@ -522,7 +522,7 @@ struct mxg_engine {
     int *d_item_ctr = nullptr;          // the force kernel's work-item counter and finished-warp count
     int *d_item_order = nullptr;        // work items, most crowded cells first (when cells are split)
     bool order_items = false;
-    long long occupancy_hint = 0;       // particle count the work-item split is decided on (0: nparts)
+    long long occupancy_hint = 0;       // particle count the kernel and the work items are decided on (0: nparts)
     bool dpd_pure = false;              // every pair potential DPD (not shifted), no summed second term
     int *d_cell_planes = nullptr;       // planes summed into each cell's forces
     int nitems = 0;
@@ -1294,8 +1294,11 @@ int mxg_engine::start(cudaStream_t st) {
     // average, and a few to spare (a warp that finds no group ends at once, one that finds several
     // takes them in turn).
     std::vector<char> by_column(spaces.size());
+    // a slab's engine has the whole grid and its own particles and ghosts: it decides on the whole box's, as for
+    // the items below, so that every slab takes the kernel that the undivided box takes
     std::vector<long long> rep_parts(spaces.size(), 0);
     for (int p : prep) ++rep_parts[p];
+    if (occupancy_hint > 0 && spaces.size() == 1) rep_parts[0] = occupancy_hint;
     std::vector<int4> hcol, hfluxcol;
     std::vector<char> hflux_columns(spaces.size(), 0);
     flux_cells = false;
