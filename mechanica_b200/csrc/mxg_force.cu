@@ -26,8 +26,10 @@
  * the kColumnSpan cells that a warp's particles may span and those on both sides of them: longer
  * columns are cut into parts of that length, so the unit is the same for every warp of a space.
  *
- * The sums' order is fixed by the column's own content, so results depend neither on scheduling nor
- * on what else is in the engine.
+ * The sums' order is fixed by the column's own content and the number of warps that share a group,
+ * so results do not depend on scheduling. That number follows the engine's particles (or a pinned
+ * variant), and the instantiation and the choice of this kernel what potentials the engine has: with
+ * all of them alike, a replica has the bits that it has alone.
  *
  * Bound: instruction issue and latency (15 to 17 warps a SM, limited by the staged particles; 54 % of
  * the issue slots). Of a DPD pass over 200,000 particles in 16,000 cells of the cutoff, by leaving phases
