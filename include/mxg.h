@@ -437,6 +437,12 @@ int mxg_engine_set_step_counter(mxg_engine *e, unsigned long long step);
  * (an A-B radial distribution) is built on it. No counterpart in the reference. */
 int mxg_rdf(const void *x4, int n, const double *box, int type_a, int type_b, int nbins, double dr, double sigma,
             void *hist, const double *coef, void *grad4, void *stream);
+/* The same with the caller's scratch (device memory, 16-byte aligned, of at least the bytes that mxg_rdf_scratch
+ * gives for the same particles, box and bins; in use until the stream has passed the call). mxg_rdf allocates
+ * and frees it on the stream, which between synchronisations costs up to tens of milliseconds a call. */
+int mxg_rdf_scratch(int n, const double *box, int nbins, double dr, double sigma, size_t *bytes);
+int mxg_rdf_in(const void *x4, int n, const double *box, int type_a, int type_b, int nbins, double dr, double sigma,
+               void *hist, const double *coef, void *grad4, void *scratch, size_t scratch_bytes, void *stream);
 
 /* The integrator (engine.h EngineIntegrator, set by universe_init from the `integrator` keyword,
  * src/MxSimulator.cpp:218-230): 0 forward Euler (engine_advance_forward_euler), 1 Runge-Kutta 4

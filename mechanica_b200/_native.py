@@ -144,6 +144,10 @@ _SIGS = {
     "mxg_engine_set_step_counter": ([_vp, ctypes.c_ulonglong], ctypes.c_int),
     "mxg_rdf": ([_vp, ctypes.c_int, _c_double_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,
                  ctypes.c_double, _vp, _vp, _vp, _vp], ctypes.c_int),
+    "mxg_rdf_scratch": ([ctypes.c_int, _c_double_p, ctypes.c_int, ctypes.c_double, ctypes.c_double,
+                         ctypes.POINTER(ctypes.c_size_t)], ctypes.c_int),
+    "mxg_rdf_in": ([_vp, ctypes.c_int, _c_double_p, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_double,
+                    ctypes.c_double, _vp, _vp, _vp, _vp, ctypes.c_size_t, _vp], ctypes.c_int),
     "mxg_potential_params": ([_vp, _c_double_p, ctypes.c_int], ctypes.c_int),
     "mxg_potential_coeffs64": ([_vp, _c_double_p, ctypes.c_int], ctypes.c_int),
     "mxg_potential_refit": ([_vp, _c_double_p, ctypes.c_int], ctypes.c_int),

@@ -199,16 +199,25 @@ def trajectory(theta, x0, v0, sim):
     return Trajectory.apply(theta, x0, v0, sim)
 
 
+def _rdf(x4, cfg, hist=None, coef=None, grad4=None):
+    """mxg_rdf with scratch from the caching allocator (the device is synchronised before it goes back)."""
+    box, ta, tb, nbins, dr, sigma, norm = cfg
+    n, boxa, need = x4.shape[0], (ctypes.c_double * 3)(*box), ctypes.c_size_t()
+    check(lib().mxg_rdf_scratch(n, boxa, nbins, dr, sigma, ctypes.byref(need)), "rdf")
+    scratch = torch.empty(max(need.value, 1), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    check(lib().mxg_rdf_in(_dptr(x4), n, boxa, ta, tb, nbins, dr, sigma, _dptr(hist) if hist is not None else None,
+                           _dptr(coef) if coef is not None else None, _dptr(grad4) if grad4 is not None else None,
+                           _dptr(scratch), scratch.numel(), None), "rdf")
+    torch.cuda.synchronize()
+
+
 class _RdfLoss(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x4, target, cfg):
         box, ta, tb, nbins, dr, sigma, norm = cfg
         hist = torch.zeros(nbins, dtype=torch.int64, device="cuda")
-        boxa = (ctypes.c_double * 3)(*box)
-        torch.cuda.synchronize()
-        check(lib().mxg_rdf(_dptr(x4), x4.shape[0], boxa, ta, tb, nbins, dr, sigma, _dptr(hist), None, None,
-                            None), "rdf")
-        torch.cuda.synchronize()
+        _rdf(x4, cfg, hist=hist)
         H = hist.to(torch.float64) / RDF_FIXED
         g = H * norm
         ctx.save_for_backward(x4, g, target)
@@ -222,12 +231,7 @@ class _RdfLoss(torch.autograd.Function):
         coef = (2.0 * (g - target) * gl + (gg if gg is not None else 0.0)) * norm
         coef = coef.contiguous()
         grad4 = torch.zeros_like(x4)
-        boxa = (ctypes.c_double * 3)(*box)
-        torch.cuda.synchronize()
-        check(lib().mxg_rdf(_dptr(x4), x4.shape[0], boxa, ta, tb, nbins, dr, sigma, None,
-                            ctypes.cast(coef.data_ptr(), ctypes.POINTER(ctypes.c_double)), _dptr(grad4), None),
-              "rdf_grad")
-        torch.cuda.synchronize()
+        _rdf(x4, ctx.cfg, coef=coef, grad4=grad4)
         return grad4, None, None
 
 

@@ -1093,14 +1093,12 @@ __global__ void __launch_bounds__(kRdfCellWarps * 32) rdf_cell_kernel(RdfGrid g,
     }
 }
 
-/* The cell grid's histogram and gradient. False when the grid does not apply: the box is less
- * than three reaches wide on an axis (a particle would meet a partner's image twice), there are too
- * few particles for the grid's launches to pay, or its scratch cannot be allocated. */
+/* The cell grid of a box, without its arrays. False when the grid does not apply: the box is less
+ * than three reaches wide on an axis (a particle would meet a partner's image twice), or there are too
+ * few particles for the grid's launches to pay. */
 constexpr int kRdfGridMin = 1024;
-bool launch_rdf_grid(const float4 *x, int n, const double *box, int ta, int tb, int nbins, double dr, double sigma,
-                     unsigned long long *hist, const double *coef, float4 *grad, int sms, cudaStream_t st) {
+bool rdf_grid(int n, const double *box, int nbins, double dr, double sigma, RdfGrid &g) {
     if (n < kRdfGridMin) return false;
-    RdfGrid g;
     const double reach = nbins * dr + 4 * sigma + kRdfMargin;
     g.ncells = 1;
     for (int k = 0; k < 3; ++k) {
@@ -1110,13 +1108,16 @@ bool launch_rdf_grid(const float4 *x, int n, const double *box, int ta, int tb, 
         g.iL[k] = 1.0 / box[k];
         g.ncells *= g.nc[k];
     }
-    // one allocation: the sorted positions first (16-byte aligned), then the integer arrays
-    const size_t ints = 3 * (size_t)n + 3 * (size_t)g.ncells + 1;
-    char *mem = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void **>(&mem), sizeof(float4) * (size_t)n + sizeof(int) * ints, st) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+    return true;
+}
+size_t rdf_grid_bytes(int n, const RdfGrid &g) {
+    return sizeof(float4) * (size_t)n + sizeof(int) * (3 * (size_t)n + 3 * (size_t)g.ncells + 1);
+}
+
+/* The histogram and gradient over grid g, its arrays in mem (rdf_grid_bytes, 16-byte aligned): the sorted
+ * positions first, then the integers. */
+void launch_rdf_grid(RdfGrid g, char *mem, const float4 *x, int n, const double *box, int ta, int tb, int nbins, double dr,
+                     double sigma, unsigned long long *hist, const double *coef, float4 *grad, int sms, cudaStream_t st) {
     g.x = reinterpret_cast<float4 *>(mem);
     g.count = reinterpret_cast<int *>(g.x + n);
     g.fill = g.count + g.ncells;
@@ -1138,9 +1139,26 @@ bool launch_rdf_grid(const float4 *x, int n, const double *box, int ta, int tb, 
         cudaMemsetAsync(grad, 0, sizeof(float4) * (size_t)n, st);  // particles of neither type
         rdf_cell_kernel<true><<<grid, kRdfCellWarps * 32, 0, st>>>(g, b3, ta, tb, nbins, dr, sigma, nullptr, coef, grad);
     }
-    cudaFreeAsync(mem, st);
-    return true;
 }
+
+/* The all-pairs kernels' split of the partner range into chunks of whole tiles, one block per (particle tile,
+ * chunk), so that a few hundred blocks (not one per SM) hide the candidate test's latency. */
+struct RdfSplit {
+    int sms, grid, chunk, nch;
+};
+RdfSplit rdf_split(int n) {
+    RdfSplit s;
+    int dev = 0;
+    s.sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&s.sms, cudaDevAttrMultiProcessorCount, dev);
+    s.grid = (n + kRdfTile - 1) / kRdfTile;
+    const int nchunks = std::max(1, std::min(s.grid, (6 * s.sms + s.grid - 1) / s.grid));
+    s.chunk = ((s.grid + nchunks - 1) / nchunks) * kRdfTile;
+    s.nch = (n + s.chunk - 1) / s.chunk;
+    return s;
+}
+size_t rdf_part_bytes(int n, const RdfSplit &s) { return sizeof(double) * 3 * (size_t)n * s.nch; }
 
 }  // namespace
 
@@ -1148,30 +1166,34 @@ void launch_positions(const EngineView &v, float4 *x_out, float4 *v_out, cudaStr
     positions_kernel<<<(v.nparts + 255) / 256, 256, 0, st>>>(v, x_out, v_out);
 }
 
+size_t rdf_scratch_bytes(int n, const double *box, int nbins, double dr, double sigma) {
+    RdfGrid g;
+    return rdf_grid(n, box, nbins, dr, sigma, g) ? rdf_grid_bytes(n, g) : rdf_part_bytes(n, rdf_split(n));
+}
+
 int launch_rdf(const float4 *x, int n, const double *box, int ta, int tb, int nbins, double dr, double sigma,
-               unsigned long long *hist, const double *coef, float4 *grad, cudaStream_t st) {
+               unsigned long long *hist, const double *coef, float4 *grad, void *scratch, cudaStream_t st) {
     if (nbins < 1 || nbins > kRdfMaxBins) return -1;
     const double3 b = make_double3(box[0], box[1], box[2]);
-    const int grid = (n + kRdfTile - 1) / kRdfTile;
-    // the partner range split into chunks of whole tiles, one block per (particle tile, chunk),
-    // so that a few hundred blocks (not one per SM) hide the candidate test's latency
-    int sms = 148, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (launch_rdf_grid(x, n, box, ta, tb, nbins, dr, sigma, hist, coef, grad, sms, st)) return 0;
-    const int ntiles = grid;
-    const int nchunks = std::max(1, std::min(ntiles, (6 * sms + grid - 1) / grid));
-    const int chunk = ((ntiles + nchunks - 1) / nchunks) * kRdfTile;
-    const int nch = (n + chunk - 1) / chunk;
-    const dim3 g2(grid, nch);
-    if (hist) rdf_hist_kernel<<<g2, kRdfTile, 0, st>>>(x, n, b, ta, tb, nbins, dr, sigma, chunk, hist);
+    const RdfSplit s = rdf_split(n);
+    RdfGrid g;
+    if (rdf_grid(n, box, nbins, dr, sigma, g)) {
+        void *mem = scratch;
+        if (mem || cudaMallocAsync(&mem, rdf_grid_bytes(n, g), st) == cudaSuccess) {
+            launch_rdf_grid(g, static_cast<char *>(mem), x, n, box, ta, tb, nbins, dr, sigma, hist, coef, grad, s.sms, st);
+            if (!scratch) cudaFreeAsync(mem, st);
+            return 0;
+        }
+        cudaGetLastError();  // without the memory for the grid, all pairs
+    }
+    const dim3 g2(s.grid, s.nch);
+    if (hist) rdf_hist_kernel<<<g2, kRdfTile, 0, st>>>(x, n, b, ta, tb, nbins, dr, sigma, s.chunk, hist);
     if (grad) {
-        double *gpart = nullptr;
-        if (cudaMallocAsync(reinterpret_cast<void **>(&gpart), sizeof(double) * 3 * (size_t)n * nch, st) != cudaSuccess)
-            return -2;
-        rdf_grad_kernel<<<g2, kRdfTile, 0, st>>>(x, n, b, ta, tb, nbins, dr, sigma, chunk, coef, gpart);
-        rdf_grad_sum_kernel<<<(n + 255) / 256, 256, 0, st>>>(gpart, n, nch, grad);
-        cudaFreeAsync(gpart, st);
+        void *gpart = scratch;
+        if (!gpart && cudaMallocAsync(&gpart, rdf_part_bytes(n, s), st) != cudaSuccess) return -2;
+        rdf_grad_kernel<<<g2, kRdfTile, 0, st>>>(x, n, b, ta, tb, nbins, dr, sigma, s.chunk, coef, static_cast<double *>(gpart));
+        rdf_grad_sum_kernel<<<(n + 255) / 256, 256, 0, st>>>(static_cast<double *>(gpart), n, s.nch, grad);
+        if (!scratch) cudaFreeAsync(gpart, st);
     }
     return 0;
 }

@@ -33,9 +33,11 @@ struct AdjointView {
 };
 
 void launch_positions(const EngineView &v, float4 *x_out, float4 *v_out, cudaStream_t st);
-/* Smoothed pair histogram of types (ta, tb) and/or its gradient (see mxg_rdf). */
+/* Smoothed pair histogram of types (ta, tb) and/or its gradient (see mxg_rdf); scratch: rdf_scratch_bytes
+ * bytes, or null to have them allocated and freed on the stream. */
+size_t rdf_scratch_bytes(int n, const double *box, int nbins, double dr, double sigma);
 int launch_rdf(const float4 *x, int n, const double *box, int ta, int tb, int nbins, double dr, double sigma,
-               unsigned long long *hist, const double *coef, float4 *grad, cudaStream_t st);
+               unsigned long long *hist, const double *coef, float4 *grad, void *scratch, cudaStream_t st);
 /* Up to kCopyMax device-to-device copies of whole 4-byte words in one launch (the sections of a
  * state snapshot): section k copies words[k] words from src[k] to dst[k]. */
 constexpr int kCopyMax = 12;

@@ -2905,18 +2905,43 @@ int mxg_engine_set_step_counter(mxg_engine *e, unsigned long long step) {
     return MXG_OK;
 }
 
-int mxg_rdf(const void *x4, int n, const double *box, int type_a, int type_b, int nbins, double dr, double sigma,
-            void *hist, const double *coef, void *grad4, void *stream) {
+namespace {
+int rdf(const void *x4, int n, const double *box, int type_a, int type_b, int nbins, double dr, double sigma, void *hist,
+        const double *coef, void *grad4, void *scratch, void *stream) {
     if (!x4 || !box || (!hist && !grad4) || (grad4 && !coef)) return MXG_ERR_NULL;
     if (n < 0 || !(dr > 0) || !(sigma > 0)) return MXG_ERR_ARG;
     if (n == 0) return MXG_OK;
     const int rc = launch_rdf(static_cast<const float4 *>(x4), n, box, type_a, type_b, nbins, dr, sigma,
-                              static_cast<unsigned long long *>(hist), coef, static_cast<float4 *>(grad4),
+                              static_cast<unsigned long long *>(hist), coef, static_cast<float4 *>(grad4), scratch,
                               static_cast<cudaStream_t>(stream));
     if (rc == -1) return MXG_ERR_RANGE;
     if (rc == -2) return MXG_ERR_MALLOC;
     CUDA_TRY(cudaGetLastError());
     return MXG_OK;
+}
+}  // namespace
+
+int mxg_rdf(const void *x4, int n, const double *box, int type_a, int type_b, int nbins, double dr, double sigma,
+            void *hist, const double *coef, void *grad4, void *stream) {
+    return rdf(x4, n, box, type_a, type_b, nbins, dr, sigma, hist, coef, grad4, nullptr, stream);
+}
+
+int mxg_rdf_scratch(int n, const double *box, int nbins, double dr, double sigma, size_t *bytes) {
+    if (!box || !bytes) return MXG_ERR_NULL;
+    if (n < 0 || !(dr > 0) || !(sigma > 0)) return MXG_ERR_ARG;
+    if (nbins < 1 || nbins > 256) return MXG_ERR_RANGE;
+    *bytes = n == 0 ? 0 : rdf_scratch_bytes(n, box, nbins, dr, sigma);
+    return MXG_OK;
+}
+
+int mxg_rdf_in(const void *x4, int n, const double *box, int type_a, int type_b, int nbins, double dr, double sigma,
+               void *hist, const double *coef, void *grad4, void *scratch, size_t scratch_bytes, void *stream) {
+    size_t need = 0;
+    const int rc = mxg_rdf_scratch(n, box, nbins, dr, sigma, &need);
+    if (rc != MXG_OK) return rc;
+    if (need > 0 && !scratch) return MXG_ERR_NULL;
+    if (scratch_bytes < need || reinterpret_cast<size_t>(scratch) % 16 != 0) return MXG_ERR_ARG;
+    return rdf(x4, n, box, type_a, type_b, nbins, dr, sigma, hist, coef, grad4, scratch, stream);
 }
 
 int mxg_engine_finalize(mxg_engine *e) {
