@@ -3,8 +3,8 @@
 TEST INFRASTRUCTURE ONLY. Computes the nonbonded forces and energy of a
 configuration in FP32 (reference operation order) or FP64 on the same FP32
 table coefficients. Tables come from the reference's own table builder
-(oracle/_ref/libmxref.so) when it is built, else from this package's builder
-(bit-identical to the committed golden tables, tests/test_tables.py).
+(oracle/_ref/libmxref.so) when it is built, else from this package's builder, each held
+to the potential's closed form (check_table).
 """
 import ctypes
 import os
@@ -83,18 +83,107 @@ def reference_table(kind, params):
                 b=b.value, r0p1=r0.value), coef
 
 
+def _closed_form(kind, params):
+    """(V(s), flags that count, first and last s, r0 + 1) of a potential's closed form in FP64, as the
+    reference's constructors state it (MxPotential.cpp:423-594, 1563-1620); s is the table's variable:
+    the distance, for Morse shifted by the radii, for power divided by their sum, for angles the cosine."""
+    q = [float(v) for v in params]
+    shifted, scaled = 1 << 12, 1 << 11
+    if kind == "lj126":
+        lo, hi, A, B, _ = q
+        return lambda r: A * r ** -12.0 - B * r ** -6.0, 0, lo, hi, None
+    if kind == "morse":
+        d, al, r0, lo, hi, _ = q
+        return lambda r: d * (np.exp(-2 * al * (r - 1)) - 2 * np.exp(-al * (r - 1))), shifted, lo, hi, r0 + 1
+    if kind == "harmonic":
+        k, r0, lo, hi, _ = q
+        return lambda r: k * (r - r0) ** 2, None, lo, hi, None
+    if kind == "power":
+        k, r0, al, lo, hi, _ = q
+        return lambda r: k * np.abs(r - r0) ** al, scaled, lo, hi, None
+    if kind == "harmonic_angle":
+        k, t0, lo, hi, _ = q
+        return (lambda c: k * (np.arccos(np.clip(c, -1, 1)) - t0) ** 2, None, np.cos(min(hi, np.pi)), np.cos(max(lo, 0.0)), None)
+    if kind == "harmonic_dihedral":
+        K, n, delta, _ = q
+        at = 1.0 if np.fmod(delta, np.pi) == 0 else 1.0 / (1.0 + np.sqrt(np.finfo(np.float32).eps))
+        return lambda c: K * (1 + np.cos(n * np.arccos(np.clip(c, -1, 1)) - delta)), None, -at, at, None
+    raise ValueError(f"no closed form of {kind}")
+
+
+def check_table(kind, params, info, coef):
+    """Raises unless the table is the potential's, by its closed form: the interval that the map gives for a
+    place holds it, its polynomial is within the tolerance the table was asked for (of the interval's largest
+    value, or of 1: the builder's own criterion at its sample points; twice that between them), and
+    the polynomial's slope within what that allows a polynomial of degree 5 (Markov: 25 / half-width)."""
+    def fail(what):
+        raise RuntimeError(f"table of {kind} {tuple(params)}: {what}")
+    if kind == "dpd":
+        if info["kind"] != 1 or info["b"] != np.float32(params[3]) or info["a"] != np.sqrt(np.finfo(np.float32).eps):
+            fail("not the DPD potential's range")
+        if bool(info["flags"] & (1 << 12)) != bool(len(params) > 4 and params[4]):
+            fail("wrong shift by the radii")
+        return
+    V, flags, lo, hi, r0p1 = _closed_form(kind, params)
+    tol = float(params[-1])
+    f32 = np.float32
+    if info["kind"] != 0 or abs(info["a"] - lo) > 1e-6 * abs(lo) or abs(info["b"] - hi) > 1e-6 * abs(hi):
+        fail(f"range {info['a']} to {info['b']}")
+    if flags is not None and info["flags"] & (3 << 11) != flags:
+        fail("wrong scaling or shift by the radii")
+    if r0p1 is not None and abs(info["r0p1"] - r0p1) > 2e-7 * max(1.0, abs(r0p1)):
+        fail(f"r0 + 1 is {info['r0p1']}")
+    c = np.asarray(coef, dtype=np.float64).reshape(-1, 8)
+    if len(c) != info["n"] + 1:
+        fail(f"{len(c)} intervals")
+    s = np.linspace(info["a"], info["b"], 32 * info["n"] + 1).astype(f32)
+    ind = _table_index(info, s)
+    s = s.astype(np.float64)
+    x = (s - c[ind, 0]) * c[ind, 1]
+    if np.abs(x).max() > 1 + 1e-3:
+        fail("the map gives intervals that do not hold their places")
+    poly = [c[ind, k] for k in range(2, 8)]
+    val, slope = poly[0], 5 * poly[0]
+    for k in range(1, 6):
+        val = val * x + poly[k]
+        slope = slope * x + (5 - k) * poly[k] if k < 5 else slope
+    want = V(s)
+    big = np.ones(len(c))
+    np.maximum.at(big, ind, np.abs(want))
+    if (np.abs(val - want) > 2 * tol * big[ind]).any():
+        fail(f"values off by {np.max(np.abs(val - want) / big[ind]):.2g} where {tol:.2g} was asked for")
+    inner = slice(1, -1)  # central differences of the closed form
+    e = 1e-6 * (info["b"] - info["a"])
+    d = (V(s[inner] + e) - V(s[inner] - e)) / (2 * e)
+    off = np.abs(slope[inner] * c[ind[inner], 1] - d) / (np.abs(c[ind[inner], 1]) * big[ind[inner]])
+    if kind not in ("harmonic_angle", "harmonic_dihedral") and (off > 25 * 2 * tol).any():
+        fail(f"slopes off by {off.max():.2g} of the interval's")
+
+
+_told = False
+
+
 def _package_table(kind, params):
-    """The same from this package's table builder, whose tables tests/test_tables.py holds bit for
-    bit to the committed golden ones (for where the reference's sources are not at hand)."""
+    """The same from this package's table builder, for where the reference's sources are not at hand. tests/
+    test_tables.py holds that builder bit for bit to the committed golden tables, for their parameters; any
+    other table is held to its closed form here, so a fault in the builder is not on both sides of a
+    comparison."""
+    global _told
     from mechanica_b200 import EngineError, workloads
+    if not _told:
+        import warnings
+        warnings.warn("oracle: tables from the package's own builder, checked against their closed forms (the reference's "
+                      "builder is not built here)", stacklevel=3)
+        _told = True
     try:
         p = workloads.make_potential(kind, [float(q) for q in params])
     except EngineError:
         return None, None
     i = p._info()
     coef = p.coefficients if i["kind"] == 0 else np.zeros(8, dtype=np.float32)
-    return dict(kind=i["kind"], flags=i["flags"], n=i["n"], alpha=i["alpha"][:3], a=i["a"], b=i["b"],
-                r0p1=i["r0_plusone"]), coef
+    info = dict(kind=i["kind"], flags=i["flags"], n=i["n"], alpha=i["alpha"][:3], a=i["a"], b=i["b"], r0p1=i["r0_plusone"])
+    check_table(kind, params, info, coef)
+    return info, coef
 
 
 def cell_origins(dim, cdim, origin=(0.0, 0.0, 0.0)):
