@@ -46,15 +46,20 @@ constexpr unsigned kFull = 0xffffffffu;
  */
 constexpr int kNearQuanta = 6;
 __device__ __forceinline__ int axis_sid(int k) { return k == 0 ? 4 : k == 1 ? 10 : 12; }  // the axes' directions
-__device__ __forceinline__ bool near_face(const DevSpace &S, int k, int kmin, int kmax) {
-    return kmin <= (int)__fmul_rn(S.sort_dscale, S.sort_bias) + kNearQuanta ||
-           kmax >= (int)__fmul_rn(S.sort_dscale, __fadd_rn(S.sort_bias, S.h[k])) - kNearQuanta;
+/* The keys up to which (w) and from which on (x, y, z) a cell's particle is near a face. */
+__device__ __forceinline__ int4 near_keys(const DevSpace &S) {
+    auto high = [&](int k) { return (int)__fmul_rn(S.sort_dscale, __fadd_rn(S.sort_bias, S.h[k])) - kNearQuanta; };
+    return make_int4(high(0), high(1), high(2), (int)__fmul_rn(S.sort_dscale, S.sort_bias) + kNearQuanta);
+}
+__device__ __forceinline__ bool near_face(const int4 &near, int k, int kmin, int kmax) {
+    return kmin <= near.w || kmax >= (k == 0 ? near.x : k == 1 ? near.y : near.z);
 }
 
 __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos, int start, int n, const DevSpace &S,
                                                  int2 *out, int *near_out) {
     const int lane = threadIdx.x & 31;
     const float bias = S.sort_bias, dscale = S.sort_dscale;
+    const int4 keys = near_keys(S);
     bool near = false;
     if (n <= 32) {  // one particle per lane
         const bool live = lane < n;
@@ -65,7 +70,7 @@ __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos,
             const int kmin = __reduce_min_sync(kFull, live ? key : 0x7fffffff);
             const int kmax = __reduce_max_sync(kFull, live ? key : -1);
             for (int k = 0; k < 3; ++k)
-                if (sid == axis_sid(k)) near |= near_face(S, k, kmin, kmax);
+                if (sid == axis_sid(k)) near |= near_face(keys, k, kmin, kmax);
             if (lane == 0) out[sid] = make_int2(kmin, kmax);
         }
         if (lane == 0) *near_out = near;
@@ -83,7 +88,7 @@ __device__ __forceinline__ void cell_sort_bounds(const float4 *__restrict__ pos,
         kmin = __reduce_min_sync(kFull, kmin);
         kmax = __reduce_max_sync(kFull, kmax);
         for (int k = 0; k < 3; ++k)
-            if (sid == axis_sid(k)) near |= near_face(S, k, kmin, kmax);
+            if (sid == axis_sid(k)) near |= near_face(keys, k, kmin, kmax);
         if (lane == 0) out[sid] = make_int2(kmin, kmax);
     }
     if (lane == 0) *near_out = near;
@@ -2273,7 +2278,12 @@ __global__ void __launch_bounds__(kThreads, 1280 / kThreads) scatter_kernel(
     __shared__ int s_mover[kScatterCells * kRow];  // ids of the buckets' movers
     __shared__ int s_kmin[kScatterCells * 13], s_kmax[kScatterCells * 13];
     __shared__ int s_start[kScatterCells], s_base[kScatterCells + 1], s_first[kScatterCells], s_in[kScatterCells];
-    __shared__ int s_rep[kScatterCells], s_net[kWarps], s_stay[2][kWarps];
+    __shared__ int s_net[kWarps], s_stay[2][kWarps];
+    // what the key bounds need of the cells' space, loaded beside the particles: the chain replica, space would
+    // otherwise stand at the kernel's end (2,000 particles in 216 cells: 11.2 us, 10.5 so)
+    __shared__ float s_bias[kScatterCells], s_dscale[kScatterCells];
+    __shared__ int4 s_near[kScatterCells];
+    __shared__ bool s_keys[kScatterCells];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int c0 = blockIdx.x << group_log2, nc = min(1 << group_log2, ncells - c0);
     const int beg = old_start[c0], end = old_start[c0 + nc - 1] + old_count[c0 + nc - 1];
@@ -2299,7 +2309,11 @@ __global__ void __launch_bounds__(kThreads, 1280 / kThreads) scatter_kernel(
         nn = on - out_count[c0 + tid] + in;
         s_start[tid] = old_start[c0 + tid];
         s_in[tid] = in;
-        s_rep[tid] = v.cell_rep[c0 + tid];
+        const DevSpace &S = v.spaces[v.cell_rep[c0 + tid]];
+        s_keys[tid] = S.prune & 2;
+        s_bias[tid] = S.sort_bias;
+        s_dscale[tid] = S.sort_dscale;
+        s_near[tid] = near_keys(S);
         clear_in[c0 + tid] = 0;
         clear_out[c0 + tid] = 0;
     }
@@ -2425,9 +2439,8 @@ __global__ void __launch_bounds__(kThreads, 1280 / kThreads) scatter_kernel(
         for (int i = g; i < nc << parts_log2; i += kGroups) {
             const int l = i >> parts_log2;
             const int b = s_base[l], e = s_base[l + 1];
-            const DevSpace &S = v.spaces[s_rep[l]];
-            if (!(S.prune & 2)) continue;
-            const float bias = S.sort_bias, dscale = S.sort_dscale;
+            if (!s_keys[l]) continue;
+            const float bias = s_bias[l], dscale = s_dscale[l];
             // the key does not fall as the projection rises: one conversion a bound. A projection that has no
             // key counts as key 0, as in cell_sort_bounds
             float lo = INFINITY, hi = -INFINITY;
@@ -2455,10 +2468,9 @@ __global__ void __launch_bounds__(kThreads, 1280 / kThreads) scatter_kernel(
     __syncthreads();
     for (int t = tid; t < nc * 13; t += kThreads)
         if (s_base[t / 13 + 1] > s_base[t / 13]) v.sort_bounds[c0 * 13 + t] = make_int2(s_kmin[t], s_kmax[t]);
-    if (tid < nc && s_base[tid + 1] > s_base[tid] && (v.spaces[s_rep[tid]].prune & 2)) {
-        const DevSpace &S = v.spaces[s_rep[tid]];
+    if (tid < nc && s_base[tid + 1] > s_base[tid] && s_keys[tid]) {
         bool near = false;
-        for (int k = 0; k < 3; ++k) near |= near_face(S, k, s_kmin[tid * 13 + axis_sid(k)], s_kmax[tid * 13 + axis_sid(k)]);
+        for (int k = 0; k < 3; ++k) near |= near_face(s_near[tid], k, s_kmin[tid * 13 + axis_sid(k)], s_kmax[tid * 13 + axis_sid(k)]);
         v.cell_near[c0 + tid] = near;
     }
     if (tid == 0) {
