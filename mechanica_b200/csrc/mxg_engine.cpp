@@ -1303,14 +1303,20 @@ int mxg_engine::start(cudaStream_t st) {
     std::vector<char> hflux_columns(spaces.size(), 0);
     flux_cells = false;
     const bool recorded = records_hold(near_ratio);
+    const double mean_groups = (double)(occupancy_hint > 0 ? occupancy_hint : (long long)nparts) / 32.0;
+    col_split = mean_groups >= 8.0 * num_sms ? 1 : mean_groups >= 2.0 * num_sms ? 4 : 8;
     // The cell kernel evaluates each pair once where the columns do it from both sides, so it keeps the
     // engines with costly pair terms while its candidates are few: cells of up to 1.34 cutoffs with 11
-    // particles or more, 8 where a DPD term draws from the Philox stream or is summed with a table (below
-    // that it waits for loads). DPD with the reference's random term is cheap enough everywhere. Cells /
-    // columns, step: DPD with Philox, 64,000 cells of 13, edge 1.0: 884 / 1004 us, edge 1.14: 951 / 921; of
-    // 9: 587 / 583; of 6: 374 / 347; of 3: 274 / 181; Morse + DPD, 32,768 in 2,197 cells: 100 / 117; Morse,
-    // 252,000 in 24 boxes, 12 to 16 a cell, edge 1.0 to 1.08: 302 / 300. Force pass: Lennard-Jones, 10 a
-    // cell, edge 1.0: 205 / 176; 20, edge 1.25: 231 / 169. The line lies above 4/3, where three or more cells
+    // particles or more; where a DPD term draws from the Philox stream, is shifted, summed with a table or beside
+    // one, 8, 3.5 or 5.5 by the warps that share a group (8, 4, 1). Below that it waits for loads. DPD with
+    // the reference's random term is cheap enough everywhere. Cells / columns, step: DPD with Philox, 64,000
+    // cells of 13, edge 1.0: 884 / 1004 us, edge 1.14: 951 / 921; 200,000 of 7.5, 6, 5, 4, 3 a cell: 160 / 200,
+    // 152 / 174, 154 / 159, 177 / 146, 208 / 140; 60,000: 65 / 92, 63 / 80, 64 / 64, 68 / 68, 74 / 63; 20,000:
+    // 43 / 51, 37 / 47, 37 / 45, 37 / 44, 41 / 43; 3,000: 31 / 31, 31 / 30, 31 / 29, 31 / 29, 28 / 27; Morse + DPD,
+    // 60,000: 80 / 98, 74 / 81, 74 / 66, 76 / 70, 82 / 68; 20,000: 51 / 53, 44 / 50, 43 / 48, 40 / 44, 45 / 42; 32,768
+    // in 2,197 cells: 100 / 117; Morse, 252,000 in 24 boxes, 12 to 16 a cell, edge 1.0 to 1.08: 302 / 300; 20,000
+    // of 10, 8, 4, 2: 46 / 42, 42 / 38, 36 / 36, 53 / 35. Force pass: Lennard-Jones, 10 a cell, edge 1.0:
+    // 205 / 176; 20, edge 1.25: 231 / 169. The line lies above 4/3, where three or more cells
     // of the cutoff always fit, so that an ensemble's replicas take one kernel: with the smallest of four
     // (629 to 2,866 particles, its edge 1.23) by columns the two launches took a step 94 us, 79 with one.
     // Engines with species fluxes stay on the cell kernel: the sums' order moves positions in the last bit,
@@ -1330,7 +1336,8 @@ int mxg_engine::start(cudaStream_t st) {
     costly = !any_dpd || costly || rng_mode != 0;
     for (size_t r = 0; r < spaces.size(); ++r) {
         const Space &sp = spaces[r];
-        const bool few_candidates = rep_parts[r] >= (any_dpd ? 8LL : 11LL) * sp.ncells && sp.h[2] < 1.34 * cutoff;
+        const long long half_line = !any_dpd ? 22 : col_split == 8 ? 16 : col_split == 4 ? 7 : 11;
+        const bool few_candidates = 2 * rep_parts[r] >= half_line * sp.ncells && sp.h[2] < 1.34 * cutoff;
         by_column[r] = recorded && !has_fluxes && (fades || costly) && sp.columns_apply(cutoff) && !(costly && few_candidates);
         const bool flux_columns = has_fluxes && sp.columns_apply(cutoff);
         hflux_columns[r] = flux_columns;
@@ -1351,8 +1358,6 @@ int mxg_engine::start(cudaStream_t st) {
     }
     ncol_items = (int)hcol.size();
     nflux_items = (int)hfluxcol.size();
-    const double mean_groups = (double)(occupancy_hint > 0 ? occupancy_hint : (long long)nparts) / 32.0;
-    col_split = mean_groups >= 8.0 * num_sms ? 1 : mean_groups >= 2.0 * num_sms ? 4 : 8;
     const bool crowded = (occupancy_hint > 0 ? occupancy_hint : (long long)nparts) >= 16LL * std::max(1, ncells);
     const int want_warps = num_sms * (crowded ? 64 : 5 * kWarpsPerBlock);
     const int parts = std::max(1, std::min(kMaxCellParts, (want_warps + ncells - 1) / std::max(1, ncells)));
