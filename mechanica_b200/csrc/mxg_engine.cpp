@@ -526,7 +526,7 @@ struct mxg_engine {
     bool dpd_pure = false;              // every pair potential DPD (not shifted), no summed second term
     int *d_cell_planes = nullptr;       // planes summed into each cell's forces
     int nitems = 0;
-    int4 *d_all_items = nullptr;        // the cell kernel's items with every cell (pair counts and virial)
+    int4 *d_all_items = nullptr;        // the cell kernel's items with every cell (pair counts and virial); may be d_items
     int nall_items = 0;
     int4 *d_col_items = nullptr;        // the column force kernel's items
     int ncol_items = 0;
@@ -1658,7 +1658,12 @@ int mxg_engine::start(cudaStream_t st) {
     rc |= alloc(&d_cell_planes, ncells);
     rc |= alloc(&d_items, hitems.size());
     rc |= alloc(&d_col_items, hcol.size());
-    rc |= alloc(&d_all_items, hall.size());
+    if (ncol_items == 0) {  // the list of the force pass is the whole one
+        hall.clear();
+        d_all_items = d_items;
+    } else {
+        rc |= alloc(&d_all_items, hall.size());
+    }
     rc |= alloc(&d_flux_items, hfluxcol.size());
     rc |= alloc(&d_item_ctr, 2);
     rc |= alloc(&d_item_order, hitems.size());
@@ -1760,7 +1765,9 @@ int mxg_engine::start(cudaStream_t st) {
         (rc = upload(d_nb_off, nb_off, stream)) || (rc = upload(d_nb_cell, nb_cell, stream)) ||
         (rc = upload(d_nb_shift, nb_shift, stream)) || (rc = upload(d_nb_rev, nb_rev, stream)) ||
         (rc = upload(d_sec_count, hsec, stream)) || (rc = upload(d_cell_planes, hplanes, stream)) ||
-        (rc = upload(d_items, hitems, stream)) || (rc = upload(d_col_items, hcol, stream)) || (rc = upload(d_all_items, hall, stream)) || (rc = upload(d_flux_items, hfluxcol, stream)) || (rc = upload(d_pots, hp, stream)) ||
+        (rc = upload(d_items, hitems, stream)) || (rc = upload(d_col_items, hcol, stream)) ||
+        (rc = upload(d_all_items, hall, stream)) || (rc = upload(d_flux_items, hfluxcol, stream)) ||
+        (rc = upload(d_pots, hp, stream)) ||
         (rc = upload(d_coef, coef, stream)) || (rc = upload(d_pot_idx, hpidx, stream)) ||
         (rc = upload(d_pot_idx2, hpidx2, stream)) || (rc = upload(d_dpd_pair, hdpd, stream)) ||
         (rc = upload(d_pair_rec, hrec, stream)) || (rc = upload(d_pair_rec2, hrec2, stream)) ||
