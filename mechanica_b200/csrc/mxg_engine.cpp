@@ -683,7 +683,7 @@ struct mxg_engine {
                 double lo, hi;
                 table_reach(pots[pidx[k]], rsum, lo, hi);
                 rec[0] = make_float4(from, scaled ? 1.0f / rsum : 1.0f, shifted ? d.r0_plusone - rsum : 0.f,
-                                     lo < 0 ? -1.f : (float)(lo * lo));
+                                     hi < 0 ? -1.f : (float)(lo * lo));
                 rec[1] = make_float4(d.alpha0, d.alpha1, d.alpha2, as_float((int)((unsigned)d.n << 20 | (unsigned)(d.coef_off / kChunk))));
                 rec[2] = make_float4(d.a2, d.b, shifted ? d.r0_plusone : 0.f, shifted ? rsum : scaled ? -rsum : 0.f);
             }
@@ -700,7 +700,8 @@ struct mxg_engine {
 
     /* The distances r between which rounding decides whether a pair is past the end of table t for types a and b
      * (radii sum rsum) or past the cutoff, whichever is nearer: the displacements' width, and a few units in
-     * the last place of what the table's variable s = m r + c is formed from. lo < 0: none is in range. */
+     * the last place of what the table's variable s = m r + c is formed from. hi < 0: none is in range. Below
+     * kClose2 every pair is left to the reference's arithmetic, so an end there starts at that distance. */
     void table_reach(const mxg::PotentialTable &t, float rsum, double &lo, double &hi) const {
         const bool scaled = t.flags & kFlagScaled, shifted = !scaled && (t.flags & kFlagShifted);
         const double m = scaled ? 1.0 / rsum : 1.0, c = shifted ? (double)t.r0_plusone - rsum : 0.0, b = t.b;
@@ -714,12 +715,15 @@ struct mxg_engine {
         const double end = (b - c) / m, w = wide + 2.4e-7 * (cutoff + (std::fabs(b) + std::fabs(c)) / m);
         lo = std::min(lo, end - w);
         hi = std::min(hi, end + w);
-        if (hi >= 0 && lo < 0) lo = 0.0;
+        const double close = std::sqrt((double)kClose2) * cutoff * (1 - 1e-6);
+        if (hi >= 0) {
+            lo = std::max(lo, close);
+            hi = std::max(hi, lo);
+        }
     }
 
-    /* Whether the records can hold every table (interval counts, places in the coefficient pool, and ends that
-     * are not so near to zero that the width around them is no small part of it); ratio: EngineView::near_ratio. */
-    bool records_hold(float &ratio) const {
+    /* EngineView::near_ratio for the tables as they are. */
+    float widest_ratio() const {
         double widest = 1.0;
         for (const Space &sp : spaces)
             for (const std::vector<int> *idx : {&sp.pot_idx, &sp.pot2_idx})
@@ -728,10 +732,13 @@ struct mxg_engine {
                     if (q < 0 || pots[q].kind == kKindDPD) continue;
                     double lo, hi;
                     table_reach(pots[q], (float)types[a].radius + (float)types[b].radius, lo, hi);
-                    if (lo >= 0 && lo < cutoff / 64) return false;
-                    if (lo >= 0) widest = std::max(widest, hi / lo);
+                    if (hi >= 0) widest = std::max(widest, hi / lo);
                 }
-        ratio = (float)(widest * widest * (1 + 2.4e-7));
+        return (float)(widest * widest * (1 + 2.4e-7));
+    }
+
+    /* Whether the records can hold every table (interval counts and places in the coefficient pool). */
+    bool records_hold() const {
         size_t intervals = 0;
         for (const auto &t : pots) {
             if (t.n >= 1 << 11) return false;
@@ -1302,7 +1309,8 @@ int mxg_engine::start(cudaStream_t st) {
     std::vector<int4> hcol, hfluxcol;
     std::vector<char> hflux_columns(spaces.size(), 0);
     flux_cells = false;
-    const bool recorded = records_hold(near_ratio);
+    const bool recorded = records_hold();
+    near_ratio = widest_ratio();
     const double mean_groups = (double)(occupancy_hint > 0 ? occupancy_hint : (long long)nparts) / 32.0;
     col_split = mean_groups >= 8.0 * num_sms ? 1 : mean_groups >= 2.0 * num_sms ? 4 : 8;
     // The cell kernel evaluates each pair once where the columns do it from both sides, so it keeps the
@@ -2203,6 +2211,13 @@ int mxg_engine_set_pot_params(mxg_engine *e, int idx, const double *params, int 
         (rc = upload(e->d_pair_rec2, hrec2, e->stream)))
         return rc;
     CUDA_TRY(cudaStreamSynchronize(e->stream));  // the host vectors go out of scope
+    // a table shifted so that it ends nearer than any did: the width around its end is a launch argument, which
+    // the step graphs hold; with room for the parameters to come
+    const float ratio = e->widest_ratio();
+    if (e->ncol_items > 0 && ratio > e->near_ratio) {
+        e->near_ratio = 1.f + 2.f * (ratio - 1.f);
+        return e->build_graphs();
+    }
     return MXG_OK;
 }
 
