@@ -1330,7 +1330,7 @@ int mxg_engine::start(cudaStream_t st) {
     // Engines with species fluxes stay on the cell kernel: the sums' order moves positions in the last bit,
     // and there that is no rounding any more. A particle that changes cells keeps its rates for a step, and one
     // pair more or less at a cutoff carries decay. 50,021 particles of 4 a cell, five entries, a step: 197 us
-    // with the forces by columns, 218 so (the fluxes themselves go by columns in both).
+    // with the forces by columns, 210 so (the fluxes themselves go by columns in both).
     // In a DPD-only pass the columns take a force at the cutoff for zero, so one that reaches further stays here.
     bool any_dpd = false, costly = false, fades = true;
     for (const Space &sp : spaces)

@@ -31,13 +31,13 @@
  * variant), and the instantiation and the choice of this kernel what potentials the engine has: with
  * all of them alike, a replica has the bits that it has alone.
  *
- * Bound: instruction issue and latency (15 to 17 warps a SM, limited by the staged particles; 54 % of
- * the issue slots). Of a DPD pass over 200,000 particles in 16,000 cells of the cutoff, by leaving phases
- * out: setting up and staging 49 us, candidates 34, pairs 50. Against the cell kernel (mxg_kernels.cu),
- * force pass: Lennard-Jones, 270,000 particles in cells of 1.0 / 1.67 / 2.5 cutoffs: 205 / 516 / 1,112
- * -> 176 / 225 / 420 us; 10,000 in the default 4^3 cells: 213 -> 63; DPD, density 3, 192,000: 165 -> 75;
- * DPD, density 13, 832,000: 551 -> 530, and 30 us less in the integrator, which has no received sums
- * to add.
+ * Bound: instruction issue and latency. A DPD pass over 200,000 particles in 16,000 cells of the cutoff: 129 us,
+ * 74.4 M warp instructions, 57 % of the issue slots, 14 warps a SM (16 by the staged particles' shared memory;
+ * profiles/column_kernel_dpd200k.md); by leaving phases out, setting up and staging 49 us, candidates 34, pairs 50.
+ * Force pass with the cell kernel (mxg_kernels.cu) / this one: Lennard-Jones, 270,000 particles in cells of
+ * 1.0 / 1.67 / 2.5 cutoffs: 204 / 511 / 1,163 -> 154 / 231 / 418 us; 10,000 in the default 4^3 cells: 208 -> 39;
+ * DPD, density 3, 192,000: 172 -> 72; density 13, 832,000: 585 -> 462, and 30 us less in the integrator, which has no
+ * received sums to add. Chains, 20,360: 40 -> 34; 3,375 DPD particles: 23 -> 15.
  */
 #include <algorithm>
 
