@@ -32,8 +32,8 @@
  * all of them alike, a replica has the bits that it has alone.
  *
  * Bound: instruction issue and latency. A DPD pass over 200,000 particles in 16,000 cells of the cutoff: 129 us,
- * 74.4 M warp instructions, 57 % of the issue slots, 14 warps a SM (16 by the staged particles' shared memory;
- * profiles/column_kernel_dpd200k.md); by leaving phases out, setting up and staging 49 us, candidates 34, pairs 50.
+ * 74.4 M warp instructions, 57 % of the issue slots, 14 warps a SM (16 by the staged particles' shared memory); by
+ * leaving phases out, setting up and staging 49 us, candidates 34, pairs 50.
  * Force pass with the cell kernel (mxg_kernels.cu) / this one: Lennard-Jones, 270,000 particles in cells of
  * 1.0 / 1.67 / 2.5 cutoffs: 204 / 511 / 1,163 -> 154 / 231 / 418 us; 10,000 in the default 4^3 cells: 208 -> 39;
  * DPD, density 3, 192,000: 172 -> 72; density 13, 832,000: 585 -> 462, and 30 us less in the integrator, which has no
